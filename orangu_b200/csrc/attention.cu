@@ -1000,60 +1000,130 @@ bool launch_attn_prefill(const AttnDecodeArgs &a, cudaStream_t st) {
 //            than a configurable bound take the flash-decode kernels above instead.
 // ====================================================================================================
 
+#include "packed.cuh"
 #include "seqsum.cuh"
 
 namespace ob {
 
 namespace {
 
-constexpr int SC_THREADS = 128;
-constexpr int SC_TILE = 64;  // positions per CTA
+// ((a0 + a4) + (a1 + a5)) + ((a2 + a6) + (a3 + a7)) of the eight running sums, held in pairs
+__device__ __forceinline__ float fold8(const uint64_t (&a)[4]) {
+    const float s0 = __fadd_rn(__fadd_rn(f2_lo(a[0]), f2_lo(a[2])), __fadd_rn(f2_hi(a[0]), f2_hi(a[2])));
+    return __fadd_rn(s0, __fadd_rn(__fadd_rn(f2_lo(a[1]), f2_lo(a[3])), __fadd_rn(f2_hi(a[1]), f2_hi(a[3]))));
+}
+// eight f16 as four pairs of fp32
+__device__ __forceinline__ void pairs8(const uint4 &h, uint64_t (&v)[4]) {
+    const uint32_t w[4] = {h.x, h.y, h.z, h.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[i]));
+        v[i] = f2_pack(f.x, f.y);
+    }
+}
+__device__ __forceinline__ void lds_pairs8(const float *p, uint64_t (&v)[4]) {
+    const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(p), b = *reinterpret_cast<const ulonglong2 *>(p + 4);
+    v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+}
 
+constexpr int SC_TILE = 32;  // positions per CTA
+
+// Single rows: grid (tiles, n_head_kv, n_rows), thread = one position of one head, all eight running sums in its registers.  The keys go
+// through shared memory: read in place, a warp's 32 positions are 32 lines a load, and that bound the kernel (17 us for 8 rows of 700).
 template <int G>
-__global__ void __launch_bounds__(SC_THREADS) attn_scores_kernel(AttnExactArgs a) {
-    extern __shared__ float sq[];  // [G][hd]
+__global__ void __launch_bounds__(SC_TILE * G) attn_scores_kernel(AttnExactArgs a) {
+    extern __shared__ __align__(16) float sq[];  // [G][hd], then the keys, rows padded by 16 bytes
     const uint32_t tile = blockIdx.x, kvh = blockIdx.y, row = blockIdx.z;
     const uint32_t n_pos = a.n_pos[row];
     const uint32_t p0 = tile * SC_TILE;
     if (p0 >= n_pos) return;
-    const uint32_t hd = a.head_dim, head0 = kvh * G;
-    for (uint32_t i = threadIdx.x; i < G * hd; i += SC_THREADS) sq[i] = a.q[(uint64_t)row * a.n_head * hd + (uint64_t)head0 * hd + i];
-    __syncthreads();
+    const uint32_t hd = a.head_dim, g = threadIdx.x / SC_TILE, p = p0 + threadIdx.x % SC_TILE, head = kvh * G + g;
+    const uint64_t ones = a.ones;
+    uint8_t *sk = reinterpret_cast<uint8_t *>(sq + G * hd);
+    const uint32_t pieces = hd / 8, pitch = hd * 2 + 16;
     const int32_t *table = a.page_tables[row];
-    const uint32_t j = threadIdx.x & 7, grp = threadIdx.x >> 3;  // 16 groups of 8 lanes
-    const uint32_t chunks = hd / 8;
+    for (uint32_t i = threadIdx.x; i < SC_TILE * pieces; i += SC_TILE * G) {
+        const uint32_t pi = i / pieces, c = i % pieces, pp = min(p0 + pi, n_pos - 1);
+        const __half *src = a.k_pool + (((uint64_t)table[pp / KV_PAGE] * a.n_head_kv + kvh) * KV_PAGE + pp % KV_PAGE) * hd + 8 * c;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(sk + pi * pitch + c * 16)), "l"(src) : "memory");
+    }
+    for (uint32_t i = threadIdx.x; i < G * hd; i += SC_TILE * G) sq[i] = a.q[((uint64_t)row * a.n_head + kvh * G) * hd + i];
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    uint64_t acc[4] = {0, 0, 0, 0};
+    const float *q = sq + g * hd;
+    const uint8_t *kp = sk + (threadIdx.x % SC_TILE) * pitch;
+#pragma unroll 4
+    for (uint32_t c = 0; c < pieces; ++c) {
+        uint64_t k[4], v[4];
+        pairs8(*reinterpret_cast<const uint4 *>(kp + c * 16), k);
+        lds_pairs8(q + 8 * c, v);
 #pragma unroll
-    for (int it = 0; it < SC_TILE / 16; ++it) {
-        const uint32_t p = p0 + grp + 16 * it;
-        const bool live = p < n_pos;  // uniform within a group of 8
-        float acc[G];
+        for (int m = 0; m < 4; ++m) acc[m] = f2_add(f2_mul(v[m], k[m]), acc[m], ones);
+    }
+    if (p < n_pos) a.scores[((uint64_t)row * a.n_head + head) * a.score_stride + p] = __fmul_rn(fold8(acc), a.scale);
+}
+
+// Consecutive rows of one sequence: grid (tiles of 64 positions, n_head_kv, tiles of 64 / G rows), 64 queries (row, head) x 64 positions in
+// shared memory as fp32, a thread 4 x 4 of them.  Two operations per product and element on the fp32 lanes are the bound: 16384 of
+// them per element of head_dim and tile.
+constexpr int SP_Q = 64, SP_P = 64;
+template <int G>
+__global__ void __launch_bounds__(256) attn_scores_span_kernel(AttnExactArgs a) {
+    constexpr uint32_t R = SP_Q / G;
+    extern __shared__ __align__(16) float smem_f[];
+    const uint32_t hd = a.head_dim, pitch = hd + 4, p0 = blockIdx.x * SP_P, kvh = blockIdx.y, r0 = blockIdx.z * R;
+    const uint32_t rows = min(R, a.n_rows - r0), n_last = a.n_pos[r0 + rows - 1];
+    if (p0 >= n_last) return;
+    float *sq = smem_f, *sk = smem_f + SP_Q * pitch;
+    for (uint32_t i = threadIdx.x; i < SP_Q * hd / 4; i += 256) {
+        const uint32_t qi = i / (hd / 4), e = i % (hd / 4) * 4;
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (qi < rows * G) v = *reinterpret_cast<const float4 *>(a.q + ((uint64_t)(r0 + qi / G) * a.n_head + kvh * G + qi % G) * hd + e);
+        *reinterpret_cast<float4 *>(sq + qi * pitch + e) = v;
+    }
+    const int32_t *table = a.page_tables[r0];
+    for (uint32_t i = threadIdx.x; i < SP_P * hd / 8; i += 256) {
+        const uint32_t pi = i / (hd / 8), e = i % (hd / 8) * 8, p = p0 + pi;
+        uint64_t v[4] = {0, 0, 0, 0};
+        if (p < n_last) pairs8(*reinterpret_cast<const uint4 *>(a.k_pool + (((uint64_t)table[p / KV_PAGE] * a.n_head_kv + kvh) * KV_PAGE + p % KV_PAGE) * hd + e), v);
+        *reinterpret_cast<ulonglong2 *>(sk + pi * pitch + e) = make_ulonglong2(v[0], v[1]);
+        *reinterpret_cast<ulonglong2 *>(sk + pi * pitch + e + 4) = make_ulonglong2(v[2], v[3]);
+    }
+    __syncthreads();
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t tq = (warp >> 1) * 16 + (lane >> 3), tp = (warp & 1) * 32 + (lane & 7);  // queries tq + 4 i, positions tp + 8 j
+    const uint64_t ones = a.ones;
+    uint64_t acc[4][4][4];
 #pragma unroll
-        for (int g = 0; g < G; ++g) acc[g] = 0.0f;
-        if (live) {
-            const __half *kp = a.k_pool + (((uint64_t)table[p / KV_PAGE] * a.n_head_kv + kvh) * KV_PAGE + p % KV_PAGE) * hd;
-            __half kv[32];  // head_dim <= 256: all loads first, so that they overlap
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (uint32_t c = 0; c < 32; ++c)
-                if (c < chunks) kv[c] = kp[8 * c + j];
+        for (int j = 0; j < 4; ++j)
 #pragma unroll
-            for (uint32_t c = 0; c < 32; ++c) {
-                if (c < chunks) {
-                    const float kf = __half2float(kv[c]);
+            for (int m = 0; m < 4; ++m) acc[i][j][m] = 0;
+    for (uint32_t c = 0; c < hd; c += 8) {
+        uint64_t q[4][4];
 #pragma unroll
-                    for (int g = 0; g < G; ++g) acc[g] = __fadd_rn(acc[g], __fmul_rn(sq[g * hd + 8 * c + j], kf));
-                }
-            }
+        for (int i = 0; i < 4; ++i) lds_pairs8(sq + (tq + 4 * i) * pitch + c, q[i]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            uint64_t k[4];
+            lds_pairs8(sk + (tp + 8 * j) * pitch + c, k);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int m = 0; m < 4; ++m) acc[i][j][m] = f2_add(f2_mul(q[i][m], k[m]), acc[i][j][m], ones);
         }
+    }
 #pragma unroll
-        for (int g = 0; g < G; ++g) {
-            acc[g] = __fadd_rn(acc[g], __shfl_xor_sync(0xffffffffu, acc[g], 4));
-            acc[g] = __fadd_rn(acc[g], __shfl_xor_sync(0xffffffffu, acc[g], 1));
-            acc[g] = __fadd_rn(acc[g], __shfl_xor_sync(0xffffffffu, acc[g], 2));
-        }
-        if (live && j == 0) {
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t qi = tq + 4 * i;
+        if (qi >= rows * G) continue;
+        const uint32_t row = r0 + qi / G, n_pos = a.n_pos[row];
+        float *s = a.scores + ((uint64_t)row * a.n_head + kvh * G + qi % G) * a.score_stride + p0;
 #pragma unroll
-            for (int g = 0; g < G; ++g) a.scores[((uint64_t)row * a.n_head + head0 + g) * a.score_stride + p] = __fmul_rn(acc[g], a.scale);
-        }
+        for (int j = 0; j < 4; ++j)
+            if (p0 + tp + 8 * j < n_pos) s[tp + 8 * j] = __fmul_rn(fold8(acc[i][j]), a.scale);
     }
 }
 
@@ -1084,76 +1154,174 @@ __global__ void __launch_bounds__(128) attn_softmax_kernel(AttnExactArgs a) {
         for (uint32_t p = threadIdx.x; p < n_pos; p += blockDim.x) s[p] = __fdiv_rn(s[p], sum);
 }
 
-// grid (hd / 16, n_head_kv, n_rows), G * 16 threads: thread (g, d) carries out[h][d] = (..((0 + w_0 v_0[d]) + w_1 v_1[d]) + ..).
-// The chain reads its operands from shared memory; the CTA brings them there a tile of 2 * threads positions at a time,
-// the next tile's global loads in flight while the current tile is being added.
+// Single rows: grid (hd / 16, n_head_kv, n_rows), G * 16 threads: thread (g, d) carries out[h][d] = (..((0 + w_0 v_0[d]) + w_1 v_1[d]) + ..).
+// The chain reads its operands from shared memory, where they arrive asynchronously, 256 positions at a time and two such tiles ahead:
+// the trip to memory is paid once, not per tile.
+constexpr uint32_t AO_P = 256;
+template <int G>
+struct AoTile {
+    __half v[AO_P][16];
+    float w[G][AO_P];
+};
 template <int G>
 __global__ void __launch_bounds__(G * 16) attn_output_kernel(AttnExactArgs a) {
-    constexpr int NT = G * 16, TILE = 2 * NT;
-    __shared__ __align__(16) __half sv[2][TILE][16];
-    __shared__ __align__(16) float sw[2][G][TILE];
+    constexpr uint32_t NT = G * 16;
+    extern __shared__ __align__(16) uint8_t ao_smem[];
+    AoTile<G> *tiles = reinterpret_cast<AoTile<G> *>(ao_smem);
     const uint32_t slice = blockIdx.x, kvh = blockIdx.y, row = blockIdx.z;
     const uint32_t n_pos = a.n_pos[row], hd = a.head_dim;
     const uint32_t tid = threadIdx.x, g = tid >> 4, d = tid & 15;
     const uint32_t head0 = kvh * G;
     const float *w0 = a.scores + ((uint64_t)row * a.n_head + head0) * a.score_stride;
     const int32_t *table = a.page_tables[row];
-    const uint32_t n_tiles = (n_pos + TILE - 1) / TILE;
-
-    uint4 rv[4];      // this thread's share of a tile: positions 2 tid, 2 tid + 1, two 16-byte halves each
-    float rw[2 * G];  // and weights tid + NT * i of head i / 2 ... see the index below
-    auto load_tile = [&](uint32_t t) {
-        const uint32_t p0 = t * TILE;
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const uint32_t p = p0 + 2 * tid + i;
-            if (p < n_pos) {
-                const uint4 *src = reinterpret_cast<const uint4 *>(a.v_pool + (((uint64_t)table[p / KV_PAGE] * a.n_head_kv + kvh) * KV_PAGE + p % KV_PAGE) * hd + slice * 16);
-                rv[2 * i] = src[0];
-                rv[2 * i + 1] = src[1];
-            } else {
-                rv[2 * i] = rv[2 * i + 1] = make_uint4(0, 0, 0, 0);
+    const uint32_t n_tiles = (n_pos + AO_P - 1) / AO_P;
+    auto cp = [](void *dst, const void *src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory"); };
+    auto fetch = [&](uint32_t t) {
+        if (t < n_tiles) {
+            AoTile<G> &tl = tiles[t & 1];
+            const uint32_t p0 = t * AO_P, n = min(AO_P, n_pos - p0);
+            for (uint32_t i = tid; i < 2 * n; i += NT) {
+                const uint32_t p = p0 + i / 2;
+                cp(&tl.v[i / 2][8 * (i & 1)], a.v_pool + (((uint64_t)table[p / KV_PAGE] * a.n_head_kv + kvh) * KV_PAGE + p % KV_PAGE) * hd + slice * 16 + 8 * (i & 1));
             }
+            const uint32_t quads = (n + 3) / 4;  // (rows of weights are padded to 64)
+            for (uint32_t i = tid; i < G * quads; i += NT) cp(&tl.w[i / quads][i % quads * 4], w0 + (uint64_t)(i / quads) * a.score_stride + p0 + i % quads * 4);
         }
-#pragma unroll
-        for (int i = 0; i < 2 * G; ++i) {  // element (head i / 2, position tid + NT * (i % 2)) of the tile's weights
-            const uint32_t p = p0 + tid + NT * (i & 1);
-            rw[i] = p < n_pos ? w0[(uint64_t)(i >> 1) * a.score_stride + p] : 0.0f;
-        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    auto store_tile = [&](int buf) {
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            *reinterpret_cast<uint4 *>(&sv[buf][2 * tid + i][0]) = rv[2 * i];
-            *reinterpret_cast<uint4 *>(&sv[buf][2 * tid + i][8]) = rv[2 * i + 1];
-        }
-#pragma unroll
-        for (int i = 0; i < 2 * G; ++i) sw[buf][i >> 1][tid + NT * (i & 1)] = rw[i];
-    };
-
+    fetch(0);
+    fetch(1);
     float o = 0.0f;
-    if (n_tiles) {
-        load_tile(0);
-        store_tile(0);
-    }
-    __syncthreads();
     for (uint32_t t = 0; t < n_tiles; ++t) {
-        const int buf = (int)(t & 1);
-        if (t + 1 < n_tiles) load_tile(t + 1);
-        const uint32_t cnt = min((uint32_t)TILE, n_pos - t * TILE);
-        for (uint32_t p = 0; p < cnt; ++p) o = __fadd_rn(o, __fmul_rn(sw[buf][g][p], __half2float(sv[buf][p][d])));
-        if (t + 1 < n_tiles) store_tile(buf ^ 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();
+        const AoTile<G> &tl = tiles[t & 1];
+        const uint32_t cnt = min(AO_P, n_pos - t * AO_P);
+        uint32_t p = 0;
+        for (; p + 8 <= cnt; p += 8) {  // the products of eight positions first, so that the chain is additions alone
+            const float4 wa = *reinterpret_cast<const float4 *>(&tl.w[g][p]), wb = *reinterpret_cast<const float4 *>(&tl.w[g][p + 4]);
+            const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+            float t8[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) t8[i] = __fmul_rn(w[i], __half2float(tl.v[p + i][d]));
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o = __fadd_rn(o, t8[i]);
+        }
+        for (; p < cnt; ++p) o = __fadd_rn(o, __fmul_rn(tl.w[g][p], __half2float(tl.v[p][d])));
+        __syncthreads();
+        fetch(t + 2);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     a.out[(uint64_t)row * a.n_head * hd + (uint64_t)(head0 + g) * hd + slice * 16 + d] = o;
 }
 
+// Consecutive rows of one sequence: grid (slices of 64 of head_dim, n_head_kv, tiles of 64 / G rows), a thread carries 4 queries x 8
+// entries through the positions, 32 at a time in shared memory.
+constexpr int SO_P = 32;
 template <int G>
-void launch_exact_g(const AttnExactArgs &a, cudaStream_t st) {
-    const uint32_t tiles = (a.max_pos + SC_TILE - 1) / SC_TILE;
-    attn_scores_kernel<G><<<dim3(tiles, a.n_head_kv, a.n_rows), SC_THREADS, (size_t)G * a.head_dim * 4, st>>>(a);
+__global__ void __launch_bounds__(128) attn_output_span_kernel(AttnExactArgs a) {
+    constexpr uint32_t R = SP_Q / G;
+    __shared__ __align__(16) float sw[SO_P][SP_Q + 4], sv[SO_P][64 + 4];
+    const uint32_t hd = a.head_dim, e0 = blockIdx.x * 64, kvh = blockIdx.y, r0 = (gridDim.z - 1 - blockIdx.z) * R;  // the longest windows first
+    const uint32_t rows = min(R, a.n_rows - r0), n_first = a.n_pos[r0], n_last = a.n_pos[r0 + rows - 1];
+    const uint32_t tid = threadIdx.x, tq = (tid >> 3) * 4, te = (tid & 7) * 8;
+    const int32_t *table = a.page_tables[r0];
+    const uint64_t ones = a.ones;
+    // this thread's share of a tile: weights of query tid / 2 at 16 positions, entries of two positions
+    const uint32_t wq = tid >> 1, wp = (tid & 1) * 16, wrow = r0 + min(wq / G, rows - 1), w_pos = a.n_pos[wrow];
+    const float *wsrc = a.scores + ((uint64_t)wrow * a.n_head + kvh * G + wq % G) * a.score_stride + wp;
+    float4 rw[4];
+    uint4 rv[2];
+    auto load = [&](uint32_t p0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t p = p0 + wp + 4 * i;
+            rw[i] = p < w_pos ? *reinterpret_cast<const float4 *>(wsrc + p0 + 4 * i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const uint32_t pi = (tid >> 3) + 16 * i, p = p0 + pi;
+            rv[i] = make_uint4(0, 0, 0, 0);
+            if (p < n_last && e0 + te < hd)
+                rv[i] = *reinterpret_cast<const uint4 *>(a.v_pool + (((uint64_t)table[p / KV_PAGE] * a.n_head_kv + kvh) * KV_PAGE + p % KV_PAGE) * hd + e0 + te);
+        }
+    };
+    uint32_t n_pos[4];
+    uint64_t o[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        n_pos[i] = a.n_pos[r0 + min((tq + i) / G, rows - 1)];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) o[i][m] = 0;
+    }
+    load(0);
+    for (uint32_t p0 = 0; p0 < n_last; p0 += SO_P) {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            sw[wp + 4 * i][wq] = rw[i].x;
+            sw[wp + 4 * i + 1][wq] = rw[i].y;
+            sw[wp + 4 * i + 2][wq] = rw[i].z;
+            sw[wp + 4 * i + 3][wq] = rw[i].w;
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            uint64_t v[4];
+            pairs8(rv[i], v);
+            float *dst = &sv[(tid >> 3) + 16 * i][te];
+            *reinterpret_cast<ulonglong2 *>(dst) = make_ulonglong2(v[0], v[1]);
+            *reinterpret_cast<ulonglong2 *>(dst + 4) = make_ulonglong2(v[2], v[3]);
+        }
+        __syncthreads();
+        if (p0 + SO_P < n_last) load(p0 + SO_P);
+        const bool whole = p0 + SO_P <= n_first;  // every row sees all of the tile
+        auto step = [&](uint32_t p, bool masked) {
+            const float4 w = *reinterpret_cast<const float4 *>(&sw[p][tq]);
+            const uint64_t w2[4] = {f2_both(w.x), f2_both(w.y), f2_both(w.z), f2_both(w.w)};
+            uint64_t v[4];
+            lds_pairs8(&sv[p][te], v);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (masked && p0 + p >= n_pos[i]) continue;
+#pragma unroll
+                for (int m = 0; m < 4; ++m) o[i][m] = f2_add(f2_mul(w2[i], v[m]), o[i][m], ones);
+            }
+        };
+        if (whole) {
+#pragma unroll 8
+            for (uint32_t p = 0; p < SO_P; ++p) step(p, false);
+        } else {
+            for (uint32_t p = 0; p < SO_P && p0 + p < n_last; ++p) step(p, true);
+        }
+    }
+    if (e0 + te >= hd) return;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (tq + i >= rows * G) continue;
+        float *dst = a.out + ((uint64_t)(r0 + (tq + i) / G) * a.n_head + kvh * G + (tq + i) % G) * hd + e0 + te;
+        *reinterpret_cast<ulonglong2 *>(dst) = make_ulonglong2(o[i][0], o[i][1]);
+        *reinterpret_cast<ulonglong2 *>(dst + 4) = make_ulonglong2(o[i][2], o[i][3]);
+    }
+}
+
+template <int G>
+void launch_exact_g(AttnExactArgs a, cudaStream_t st) {
+    a.ones = F2_ONES;
+    const uint32_t row_tiles = (a.n_rows + SP_Q / G - 1) / (SP_Q / G);
+    const size_t span_smem = (size_t)(SP_Q + SP_P) * (a.head_dim + 4) * 4;
+    // rows that share their keys are worth a tile once there are half a tile of them
+    static PerDeviceOnce once;
+    const bool span = a.one_sequence && 2 * a.n_rows >= SP_Q / G &&
+                      once.run([] { return cudaFuncSetAttribute(attn_scores_span_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (SP_Q + SP_P) * (256 + 4) * 4); }) == cudaSuccess;
+    if (span) attn_scores_span_kernel<G><<<dim3((a.max_pos + SP_P - 1) / SP_P, a.n_head_kv, row_tiles), 256, span_smem, st>>>(a);
+    else attn_scores_kernel<G><<<dim3((a.max_pos + SC_TILE - 1) / SC_TILE, a.n_head_kv, a.n_rows), SC_TILE * G, (size_t)G * a.head_dim * 4 + SC_TILE * (a.head_dim * 2 + 16), st>>>(a);
     attn_softmax_kernel<<<dim3(a.n_head, a.n_rows), 128, 0, st>>>(a);
-    attn_output_kernel<G><<<dim3(a.head_dim / 16, a.n_head_kv, a.n_rows), G * 16, 0, st>>>(a);
+    if (span) attn_output_span_kernel<G><<<dim3((a.head_dim + 63) / 64, a.n_head_kv, row_tiles), 128, 0, st>>>(a);
+    else {
+        static PerDeviceOnce once_rows;
+        if (once_rows.run([] { return cudaFuncSetAttribute(attn_output_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * sizeof(AoTile<G>)); }) != cudaSuccess) return;
+        attn_output_kernel<G><<<dim3(a.head_dim / 16, a.n_head_kv, a.n_rows), G * 16, 2 * sizeof(AoTile<G>), st>>>(a);
+    }
 }
 
 }  // namespace

@@ -228,6 +228,8 @@ struct AttnExactArgs {
     uint32_t n_rows, n_head, n_head_kv, head_dim;
     float scale;
     uint32_t max_pos;          // upper bound of n_pos over the rows (sizes the score grid)
+    bool one_sequence = false; // the rows are consecutive tokens of one sequence
+    uint64_t ones;             // filled in by the launcher (packed.cuh)
 };
 OB_QUANT void launch_attn_exact(const AttnExactArgs &a, cudaStream_t st);
 OB_QUANT bool attn_exact_supported(uint32_t n_head, uint32_t n_head_kv, uint32_t head_dim);

@@ -344,6 +344,7 @@ bool run_attention(ob_model *m, uint32_t li, uint32_t T, bool exact_attn, uint32
         at.head_dim = hd;
         at.scale = 1.0f / sqrtf((float)hd);  // llama.rs:823
         at.max_pos = pos_bound;
+        at.one_sequence = one_sequence;
         launch_attn_exact(at, st);
         m->ctx->launches += 3;
         return false;
