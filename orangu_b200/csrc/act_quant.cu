@@ -114,12 +114,26 @@ __global__ void __launch_bounds__(QT) quantize_kernel(QuantArgs a) {
                 qv[i] = quantize_value(v[i], inv);
                 s8 += qv[i];
             }
-            int s16 = s8 + __shfl_xor_sync(0xffffffffu, s8, 1);
+            const int s16 = s8 + __shfl_xor_sync(0xffffffffu, s8, 1), s32 = s16 + __shfl_xor_sync(0xffffffffu, s16, 2);
             if (live) {
                 uint32_t lo = (qv[0] & 0xff) | ((qv[1] & 0xff) << 8) | ((qv[2] & 0xff) << 16) | ((uint32_t)(qv[3] & 0xff) << 24);
                 uint32_t hi = (qv[4] & 0xff) | ((qv[5] & 0xff) << 8) | ((qv[6] & 0xff) << 16) | ((uint32_t)(qv[7] & 0xff) << 24);
                 *reinterpret_cast<uint2 *>(buf.q + (uint64_t)row * buf.dim_cap + c * 8) = make_uint2(lo, hi);
                 if ((c & 1) == 0) buf.sums[(uint64_t)row * (buf.dim_cap / 16) + c / 2] = (int16_t)s16;
+                if (mode == 0 && buf.h) {
+                    auto two = [&](int i, int j) {
+                        const __half2 v = __floats2half2_rn((float)qv[i], (float)qv[j]);
+                        return *reinterpret_cast<const uint32_t *>(&v);
+                    };
+                    *reinterpret_cast<uint4 *>(buf.h + (uint64_t)row * buf.dim_cap + c * 8) = make_uint4(two(0, 2), two(1, 3), two(4, 6), two(5, 7));
+                    if ((c & 3) == 0) {
+                        const int lo = ((s32 + 32) & 63) - 32;
+                        __half *hs = buf.hs + (uint64_t)row * (buf.dim_cap / 16) + c / 32 * 16 + (c & 31) / 4;
+                        hs[0] = __int2half_rn(lo);
+                        hs[8] = __int2half_rn((s32 - lo) / 64);
+                    }
+                    if (lane == 0) buf.dt[(uint64_t)(c / 32) * buf.dt_pitch + row] = scale;
+                }
                 if (mode == 0) {
                     if (lane == 0) buf.d[(uint64_t)row * (buf.dim_cap / 256) + c / 32] = scale;
                 } else {
@@ -132,8 +146,10 @@ __global__ void __launch_bounds__(QT) quantize_kernel(QuantArgs a) {
 
 }  // namespace
 
-void launch_quantize(int source, const QuantArgs &a, cudaStream_t st) {
+void launch_quantize(int source, const QuantArgs &args, cudaStream_t st) {
+    QuantArgs a = args;
     if (a.n_rows == 0) return;
+    if (a.n_rows < ACT_H_ROWS) a.k.h = nullptr;
     switch (source) {
     case ACT_PLAIN: quantize_kernel<ACT_PLAIN><<<a.n_rows, QT, 0, st>>>(a); break;
     case ACT_RMSNORM: {

@@ -102,7 +102,7 @@ void ob_destroy(ob_ctx *ctx) {
     if (!ctx) return;
     Bind b(ctx);
     cudaStreamSynchronize(ctx->stream);
-    for (Scratch *s : {&ctx->sx, &ctx->sy, &ctx->sq, &ctx->sd, &ctx->ss, &ctx->saux, &ctx->saux2, &ctx->saux3})
+    for (Scratch *s : {&ctx->sx, &ctx->sy, &ctx->sq, &ctx->sd, &ctx->ss, &ctx->sh, &ctx->shs, &ctx->sdt, &ctx->saux, &ctx->saux2, &ctx->saux3})
         if (s->p) cudaFree(s->p);
     cudaEventDestroy(ctx->ev0);
     cudaEventDestroy(ctx->ev1);
@@ -150,7 +150,8 @@ int make_weight(ob_ctx *ctx, const uint8_t *raw, uint64_t row_bytes, uint32_t ty
     d.row_stride = (row_size + 15) & ~(uint64_t)15;
     w->bytes = d.row_stride * n_rows;
     void *mem = nullptr;
-    cudaError_t e = cudaMalloc(&mem, w->bytes);
+    const uint64_t wide_bytes = d.type == TYPE_Q4_K ? ((uint64_t)n_rows + 3) / 4 * 4 : 0;  // (and as many words for the rows' numbers)
+    cudaError_t e = cudaMalloc(&mem, w->bytes + 5 * wide_bytes);
     if (e != cudaSuccess) {
         delete w;
         return fail(ctx, OB_ERR_OOM, std::string("weight: cudaMalloc: ") + cudaGetErrorString(e));
@@ -175,7 +176,26 @@ int make_weight(ob_ctx *ctx, const uint8_t *raw, uint64_t row_bytes, uint32_t ty
     if (d.row_stride != row_size) cudaMemsetAsync(mem, 0, w->bytes, ctx->stream);
     launch_repack(src_dev, row_bytes, type, 0, col0 / be, d, ctx->stream);
     ctx->launches++;
-    e = cudaStreamSynchronize(ctx->stream);
+    if (wide_bytes) {
+        uint8_t *wide = static_cast<uint8_t *>(mem) + w->bytes;
+        cudaMemsetAsync(wide, 0, wide_bytes, ctx->stream);
+        launch_q4k_wide(d, wide, ctx->stream);
+        ctx->launches++;
+        d.wide = wide;
+        std::vector<uint8_t> flags(n_rows);
+        std::vector<uint32_t> rows;
+        e = cudaMemcpyAsync(flags.data(), wide, n_rows, cudaMemcpyDeviceToHost, ctx->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        if (e == cudaSuccess) {
+            for (uint32_t r = 0; r < n_rows; ++r)
+                if (flags[r]) rows.push_back(r);
+            d.n_wide = (uint32_t)rows.size();
+            d.wide_rows = reinterpret_cast<const uint32_t *>(wide + wide_bytes);
+            if (d.n_wide) e = cudaMemcpyAsync(wide + wide_bytes, rows.data(), rows.size() * 4, cudaMemcpyHostToDevice, ctx->stream);
+        }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);  // the vectors go
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (staging) cudaFree(staging);
     if (e != cudaSuccess) {
@@ -247,6 +267,15 @@ int quantize_for(ob_ctx *ctx, const float *x_dev, uint32_t n_tokens, uint32_t in
     act->d = static_cast<float *>(ctx->sd.p);
     act->sums = static_cast<int16_t *>(ctx->ss.p);
     act->dim_cap = in_dim;
+    if (type == TYPE_Q4_K && n_tokens >= ACT_H_ROWS) {
+        act->dt_pitch = (n_tokens + 3) / 4 * 4;
+        if ((rc = ensure(ctx, ctx->sh, (size_t)n_tokens * in_dim * 2))) return rc;
+        if ((rc = ensure(ctx, ctx->shs, (size_t)n_tokens * (in_dim / 16) * 2))) return rc;
+        if ((rc = ensure(ctx, ctx->sdt, (size_t)(in_dim / 256) * act->dt_pitch * 4))) return rc;
+        act->h = static_cast<__half *>(ctx->sh.p);
+        act->hs = static_cast<__half *>(ctx->shs.p);
+        act->dt = static_cast<float *>(ctx->sdt.p);
+    }
     QuantArgs qa{};
     qa.x = x_dev;
     qa.n_rows = n_tokens;

@@ -118,6 +118,28 @@ __global__ void dequant_rows_kernel(DevWeight w, uint32_t first_row, uint32_t n_
     out[idx] = dequant_element(w, first_row + r, e);
 }
 
+__global__ void q4k_wide_kernel(DevWeight w, uint8_t *wide) {
+    const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx < (uint64_t)w.out_dim * w.nb) {
+        uint32_t sum = 0;
+        const uint8_t *blk = w.data + (idx / w.nb) * w.row_stride + (idx % w.nb) * 144;
+        const uint4 hd = *reinterpret_cast<const uint4 *>(blk);
+        const uint32_t sc[2] = {hd.y & 0x3f3f3f3fu, (hd.w & 0x0f0f0f0fu) | ((hd.y >> 2) & 0x30303030u)};  // engine/quant.rs:653-662
+        for (int g = 0; g < 4; ++g) {
+            const uint4 a = *reinterpret_cast<const uint4 *>(blk + 16 + 32 * g), b = *reinterpret_cast<const uint4 *>(blk + 32 + 32 * g);
+            const uint32_t v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            uint32_t lo = 0, hi = 0;
+            for (int i = 0; i < 8; ++i) {
+                lo = __dp4a(v[i] & 0x0f0f0f0fu, 0x01010101u, lo);
+                hi = __dp4a((v[i] >> 4) & 0x0f0f0f0fu, 0x01010101u, hi);
+            }
+            const uint32_t s = sc[g >> 1] >> (16 * (g & 1));
+            sum += (s & 0xffu) * lo + ((s >> 8) & 0xffu) * hi;
+        }
+        if (sum > Q4K_SUM24) wide[idx / w.nb] = 1;
+    }
+}
+
 // Embedding lookup: out[t] = dequantised row tokens[t]  (llama.rs:608-614)
 __global__ void embed_kernel(DevWeight w, const uint32_t *__restrict__ tokens, uint32_t n_tokens, float *__restrict__ out) {
     uint32_t t = blockIdx.y;
@@ -129,6 +151,11 @@ __global__ void embed_kernel(DevWeight w, const uint32_t *__restrict__ tokens, u
 void launch_repack(const uint8_t *src, uint64_t src_row_bytes, uint32_t src_type, uint32_t row0, uint32_t blk0, const DevWeight &w, cudaStream_t st) {
     uint64_t total = (uint64_t)w.out_dim * w.nb;
     repack_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(src, src_row_bytes, src_type, row0, blk0, w);
+}
+
+void launch_q4k_wide(const DevWeight &w, uint8_t *wide, cudaStream_t st) {
+    const uint64_t total = (uint64_t)w.out_dim * w.nb;
+    q4k_wide_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(w, wide);
 }
 
 void launch_dequant_rows(const DevWeight &w, uint32_t first_row, uint32_t n_rows, float *out, cudaStream_t st) {

@@ -15,6 +15,8 @@
 // status word, makes all roles leave their loops, and the CTA frees its tensor memory and returns.
 #include "common.cuh"
 #include "kernels.h"
+#include "packed.cuh"
+#include "pdl.cuh"
 #include "tc5_common.cuh"
 
 namespace ob {
@@ -168,265 +170,461 @@ gemm_tc5_q8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 }
 
 // ---- Q4_K -----------------------------------------------------------------------------------------------------------
-// The 4-bit codes cannot go to the tensor core as they are: every 32-element sub-block has its own 6-bit scale, and
-// isum = sum_j sc_j * dot32_j has to be exact.  So the scale is folded into the operand, in two digits that keep every
-// product inside a byte: sc = 8 * sc_hi + sc_lo (both 0..7), code * digit <= 105, and
-//     isum = 8 * dot(code * sc_hi, x) + dot(code * sc_lo, x),      imin = dot(m_j(i), x)
-// (the min term sum_j m_j * bsum_j is itself a dot product with the sub-block's min as the "weight" of each of its
-// elements).  Eight expander warps turn each half super-block of 128 rows (TMA-loaded GGUF blocks) into those three
-// unsigned-byte planes in the swizzled operand layout -- a packed 32-bit multiply scales four codes at once -- the MMA
-// thread accumulates each plane over the super-block's eight K = 32 steps in its own tensor-memory accumulator, and the
-// epilogue warps form the super-block's fp32 term per (row, token) in the CPU's association and order:
+// The codes cannot go to the tensor core as they are: every 32-element sub-block has its own 6-bit scale, and
+// isum = sum_j sc_j * dot32_j has to be exact.  So the scale goes into the operand: sc * code <= 63 * 15 = 945 is a whole number that
+// f16 holds exactly, and so is every 8-bit activation code; fp32 accumulators add whole numbers exactly below 2^24.  Where the scales
+// times codes of every block of a row add up to no more than Q4K_SUM24, 256 products stay below that whatever the activations are, and the
+// accumulator is (float)isum.  The few rows with a larger block (two or three in a matrix of 14336; found at registration) are left to a
+// kernel of their own (gemm_few.cu); a matrix with many keeps the halves of a super-block in two accumulators, whose rounded sum is
+// (float)isum.  The min term imin = sum_j m_j * bsum_j is one K = 16 step: with bsum = lo + 64 hi, weights [m | 64 m] against [lo | hi],
+// all whole numbers that f16 holds.  The epilogue forms the super-block's fp32 term in the CPU's association and order:
 //   decode order   acc += ad * (d * isum - dmin * imin)                          (engine/vecdot.rs:3152-3178)
 //   prefill order  first for every super-block acc -= (ad * dmin) * imin, then acc += ad * (d * isum)
-//                  (engine/vecdot.rs:2119-2143, 2213-2255): two sweeps over K in one launch, the first over the block
-//                  headers only (min plane), the accumulators staying in registers.
-constexpr int K4_RING = 8;
-constexpr int K4_EXP_WARPS = 4;
-constexpr int K4_TMA_WARP = 12, K4_MMA_WARP = 13;
-constexpr int K4_THREADS = 14 * 32;
-constexpr uint32_t K4_RAW_BYTES = TC_M * 144, K4_PLANE_BYTES = TC_M * 128;
-// N: tokens per CTA tile.  The tensor core fetches its operands from shared memory at a fixed rate, so an MMA's time goes
-// with (128 + N) * 32 bytes rather than with its 128 * N * 32 multiply-adds: 128 tokens per tile amortise the three planes
-// of the weights over twice the work of 64.  Tensor memory (512 columns) holds planes * N columns per accumulator buffer:
-// two buffers for the prefill order (two planes at most), one for the decode order at N = 128 (three planes).
-template <int N>
-struct K4Smem {
-    static constexpr uint32_t IN_STAGES = N == 64 ? 3 : 2;
-    static constexpr uint32_t B_BYTES = 2 * N * 128;
-    static constexpr uint32_t RAW = 0, B = RAW + IN_STAGES * K4_RAW_BYTES;          // a raw stage is 18 KB: B stays 1024-byte aligned
-    static constexpr uint32_t PLANES = B + IN_STAGES * B_BYTES;                     // [2 stages][3 planes][128 x 128]
-    static constexpr uint32_t XD = PLANES + 2 * 3 * K4_PLANE_BYTES;                  // [ring][N] token scales
-    static constexpr uint32_t DD = XD + K4_RING * N * 4;                             // [ring][128] d | dmin << 16
-    static constexpr uint32_t BAR = DD + K4_RING * TC_M * 4;
-    static constexpr uint32_t IN_FULL = BAR, IN_EMPTY = IN_FULL + 32, PL_FULL = IN_EMPTY + 32, PL_EMPTY = PL_FULL + 16, ACC_FULL = PL_EMPTY + 16,
-                              ACC_EMPTY = ACC_FULL + 16, SLOT = ACC_EMPTY + 16, ABORT = SLOT + 8;
-    static constexpr uint32_t BYTES = ABORT + 8, ALLOC = BYTES + 1024;
-};
-static_assert(K4_RAW_BYTES % 1024 == 0, "operand tiles must stay 1024-byte aligned");
-static_assert(K4Smem<128>::ALLOC <= 227 * 1024 && K4Smem<64>::ALLOC <= 227 * 1024, "shared memory plan does not fit");
-
-struct TcK4Args {
-    GemvSegment seg;
-    GemvSegment seg2;      // a second matrix of the same type and width served by the same launch (tiles0 < gridDim.x), e.g. ffn_up next to ffn_gate
-    uint32_t tiles0;       // row tiles of `seg`; CTAs with blockIdx.x >= tiles0 work on seg2
-    const float *act_d;    // [token][pitch] per-256 activation scales
-    uint32_t act_d_pitch;
-    uint32_t n_tokens, nb;
-};
-
+//                  (engine/vecdot.rs:2119-2143, 2213-2255): two sweeps over K, the first over the block headers only.
+//
+// A CTA is persistent over tiles of 128 rows x N tokens.  Its warps: 0-7 epilogue (thread = one row x N / 2 tokens, two at a time in
+// packed fp32), 8-15 expanders (thread = half a super-block of one row), 16 loads (TMA), 17 issues products.  An expander turns its half
+// into 64 words of two f16 -- codes enter a mantissa by a mask, one packed multiply-add takes the offset off and the scale on -- and writes
+// them to tensor memory, where the products read their A operand: expanded weights never touch shared memory, whose bandwidth the
+// activations (B, f16 from the quantizer) already take.  The order of elements within a group of four is the one the mask leaves
+// (0, 2, 1, 3); the quantizer writes activations in that order.
+//
+// The form before had byte planes of the weights' scale digits in shared memory, int8 products and two or three accumulators to read
+// back: 14336 x 4096 with 512 tokens 213 us in prefill order (now 132), 4096 x 14336 with 64 tokens 70 us in decode order on mma.sync
+// tiles (now 55).  What bounds this form is instruction issue: five warps share a scheduler, and a super-block's expansion, epilogue and
+// product issue are some 250 instructions each.
+constexpr int KQ_EPI_WARPS = 8, KQ_EXP_WARPS = 8, KQ_TMA_WARP = 16, KQ_MMA_WARP = 17, KQ_THREADS = 18 * 32;
+constexpr uint32_t KQ_RAW_BYTES = TC_M * 144, KQ_A_COLS = 128;
+// TWO: the halves of a super-block have accumulators of their own (matrices with many wide rows).
 template <bool GEMM, int N>
-__global__ void __launch_bounds__(K4_THREADS, 1)
-gemm_tc5_q4k_kernel(const __grid_constant__ CUtensorMap tm_raw0, const __grid_constant__ CUtensorMap tm_hdr0, const __grid_constant__ CUtensorMap tm_raw1,
-                    const __grid_constant__ CUtensorMap tm_hdr1, const __grid_constant__ CUtensorMap tm_x, TcK4Args a) {
-    using S = K4Smem<N>;
-    constexpr uint32_t IN_STAGES = S::IN_STAGES;
-    constexpr uint32_t MAX_PLANES = GEMM ? 2 : 3, ACC_STRIDE = MAX_PLANES * N, NBUF = 2 * ACC_STRIDE <= 512 ? 2 : 1;
-    constexpr int TPT = N / 2;  // tokens per epilogue thread
+struct KqPlan {
+    static constexpr uint32_t A_COL = GEMM ? 256 : 240, MIN_COL = A_COL + 2 * KQ_A_COLS;  // tensor memory: accumulators, then the two A buffers (decode order: and their mins)
+    static constexpr uint32_t SLOT_COLS = (GEMM ? 1 : 2) * N;  // accumulators of a super-block (decode order: and of its mins), or of half of a wide one
+    static_assert(2 * SLOT_COLS <= A_COL, "products of a super-block run while the epilogue reads the one before");
+    static constexpr uint32_t B_BYTES = N * 512, B_STAGE = B_BYTES + (GEMM ? 0 : N * 128);  // decode order: and the sums of four super-blocks
+    static constexpr uint32_t B_STAGES = N > 64 ? 2 : 3, RAW_STAGES = N > 64 ? 3 : 4;
+    static constexpr uint32_t RAW = 0, B = RAW + RAW_STAGES * KQ_RAW_BYTES, BAR = B + B_STAGES * B_STAGE;
+    static constexpr uint32_t RAW_FULL = BAR, RAW_EMPTY = RAW_FULL + 8 * RAW_STAGES, B_FULL = RAW_EMPTY + 8 * RAW_STAGES, B_EMPTY = B_FULL + 8 * B_STAGES, A_FULL = B_EMPTY + 8 * B_STAGES,
+                              A_EMPTY = A_FULL + 16, XD_FULL = A_EMPTY + 16, XD_EMPTY = XD_FULL + 16, ACC_FULL = XD_EMPTY + 16, ACC_EMPTY = ACC_FULL + 16, SLOT = ACC_EMPTY + 16, ABORT = SLOT + 8;
+    static constexpr uint32_t XD = (ABORT + 8 + 127) / 128 * 128;  // token scales of a tile, [nb][N] floats; twice when there is room
+    __host__ __device__ static constexpr uint32_t xd_bytes(uint32_t nb) { return (nb * N * 4 + 127) / 128 * 128; }
+    static constexpr uint32_t bytes(uint32_t nb, uint32_t n_xd) { return XD + n_xd * xd_bytes(nb) + 1024; }
+};
+
+struct KqMaps {
+    CUtensorMap raw[3], x, bs, xd;
+};
+struct KqArgs {
+    GemvSegment seg[3];  // matrices of one width that read the same activations
+    uint32_t tiles[3];   // running sums of their row tiles
+    uint32_t n_tokens, nb, tok_tiles, n_tiles, n_xd;
+    uint64_t ones;       // F2_ONES
+};
+
+__device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t v;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(v) : "r"(a), "r"(b), "r"(c));
+    return v;
+}
+__device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b) {
+    uint32_t v;
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(v) : "r"(a), "r"(b));
+    return v;
+}
+__device__ __forceinline__ uint32_t h2_sub(uint32_t a, uint32_t b) {
+    uint32_t v;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(v) : "r"(a), "r"(b));
+    return v;
+}
+constexpr uint32_t H2_1024 = 0x64006400u, H2_M1024 = 0xe400e400u, H2_M64 = 0xd400d400u, H2_64 = 0x54005400u, H2_16TH = 0x2c002c00u;
+
+// STEPS products of K = 16 in a row: A in tensor memory (128 lanes, two f16 of K a column, 8 columns a step), B in shared memory in boxes of
+// four steps, box_step (16-byte units) apart.  One lane of a converged warp issues all of them.
+__device__ __forceinline__ void umma_f16_ta_8(uint32_t d, uint32_t a, uint64_t b, uint32_t box_step, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q, t;\n\t.reg .b64 b1, b2, b3, b4, b5, b6, b7, bs;\n\t.reg .b32 a1, a2, a3, a4, a5, a6, a7;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %5, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+        "cvt.u64.u32 bs, %3;\n\tadd.s64 b1, %2, 2;\n\tadd.s64 b2, %2, 4;\n\tadd.s64 b3, %2, 6;\n\tadd.s64 b4, %2, bs;\n\tadd.s64 b5, b4, 2;\n\tadd.s64 b6, b4, 4;\n\tadd.s64 b7, b4, 6;\n\t"
+        "add.s32 a1, %1, 8;\n\tadd.s32 a2, %1, 16;\n\tadd.s32 a3, %1, 24;\n\tadd.s32 a4, %1, 32;\n\tadd.s32 a5, %1, 40;\n\tadd.s32 a6, %1, 48;\n\tadd.s32 a7, %1, 56;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %4, p;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %4, t;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %4, t;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %4, t;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a4], b4, %4, t;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a5], b5, %4, t;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a6], b6, %4, t;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a7], b7, %4, t;\n\t}" ::"r"(d),
+        "r"(a), "l"(b), "r"(box_step), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__host__ __device__ constexpr uint32_t umma_idesc_f16(uint32_t n) { return (1u << 4) | ((n >> 3) << 17) | ((128u >> 4) << 24); }  // fp32 accumulator, A and B f16, both K-major
+
+// A counter through a ring of S places: the place and the parity of its current round.
+template <uint32_t S>
+struct Ring {
+    uint32_t at = 0, round = 0;
+    __device__ __forceinline__ void next() {
+        if (++at == S) {
+            at = 0;
+            ++round;
+        }
+    }
+    __device__ __forceinline__ uint32_t full_parity() const { return round & 1u; }
+    __device__ __forceinline__ uint32_t empty_parity() const { return (round & 1u) ^ 1u; }  // of the round before
+};
+
+// 8 words: the mins of a super-block, m_j in pairs, then 64 m_j.
+__device__ __forceinline__ void kq_mins(const uint4 &hd, uint32_t *out) {
+    const uint32_t ml = hd.z & 0x3f3f3f3fu, mh = ((hd.w >> 4) & 0x0f0f0f0fu) | ((hd.z >> 2) & 0x30303030u);
+    out[0] = h2_sub(__byte_perm(ml, 0x64646464u, 0x4140), H2_1024);
+    out[1] = h2_sub(__byte_perm(ml, 0x64646464u, 0x4342), H2_1024);
+    out[2] = h2_sub(__byte_perm(mh, 0x64646464u, 0x4140), H2_1024);
+    out[3] = h2_sub(__byte_perm(mh, 0x64646464u, 0x4342), H2_1024);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) out[4 + i] = h2_mul(out[i], H2_64);
+}
+
+template <bool GEMM, bool TWO, int N>
+__global__ void __launch_bounds__(KQ_THREADS, 1) gemm_tc5_q4k_kernel(const __grid_constant__ KqMaps maps, const __grid_constant__ KqArgs a) {
+    using P = KqPlan<GEMM, N>;
+    constexpr int TPT = N / 2;                   // tokens per epilogue thread
+    constexpr int CH = TPT % 16 || TPT >= 48 ? 8 : 16;         // tokens at a time
     extern __shared__ uint8_t smem_raw[];
     const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *smem = smem_raw + (sbase - smem_u32(smem_raw));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // two matrices in one launch fill the last wave better than two launches: 2 x 448 CTAs are 6.05 waves of 148, not 2 x 4
-    const bool second = blockIdx.x >= a.tiles0;
-    const CUtensorMap &tm_raw = second ? tm_raw1 : tm_raw0, &tm_hdr = second ? tm_hdr1 : tm_hdr0;
-    const GemvSegment &seg = second ? a.seg2 : a.seg;
-    const uint32_t row0 = (blockIdx.x - (second ? a.tiles0 : 0u)) * TC_M, tok0 = blockIdx.y * N;
-    volatile uint32_t *abort = reinterpret_cast<volatile uint32_t *>(smem + S::ABORT);
-    const uint32_t nb = a.nb;
-    const uint32_t n_visits = GEMM ? 2 * nb : nb;  // super-block visits; in the prefill order the first nb are the min sweep
-    // planes of a visit: decode order lo, hi, min; prefill order min alone, then lo, hi
-    auto n_planes = [&](uint32_t u) -> uint32_t { return GEMM ? (u < nb ? 1u : 2u) : 3u; };
+    volatile uint32_t *abort = reinterpret_cast<volatile uint32_t *>(smem + P::ABORT);
+    const uint32_t nb = a.nb, n_min = GEMM ? (nb + 15) / 16 : 0;  // prefill order: sixteen super-blocks of mins fill an A buffer
 
     if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < IN_STAGES; ++s) {
-            mbar_init(sbase + S::IN_FULL + 8 * s, 1);
-            mbar_init(sbase + S::IN_EMPTY + 8 * s, 1 + K4_EXP_WARPS);  // MMA completion (activations) + the expanders (blocks)
+        for (uint32_t i = 0; i < P::RAW_STAGES; ++i) {
+            mbar_init(sbase + P::RAW_FULL + 8 * i, 1);
+            mbar_init(sbase + P::RAW_EMPTY + 8 * i, KQ_EXP_WARPS);
         }
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(sbase + S::PL_FULL + 8 * b, K4_EXP_WARPS);
-            mbar_init(sbase + S::PL_EMPTY + 8 * b, 1);
-            mbar_init(sbase + S::ACC_FULL + 8 * b, 1);
-            mbar_init(sbase + S::ACC_EMPTY + 8 * b, TC_EPI_WARPS);
+        for (uint32_t i = 0; i < P::B_STAGES; ++i) {
+            mbar_init(sbase + P::B_FULL + 8 * i, 1);
+            mbar_init(sbase + P::B_EMPTY + 8 * i, 1);
+        }
+        for (uint32_t i = 0; i < 2; ++i) {
+            mbar_init(sbase + P::A_FULL + 8 * i, KQ_EXP_WARPS);
+            mbar_init(sbase + P::A_EMPTY + 8 * i, 1);
+            mbar_init(sbase + P::XD_FULL + 8 * i, 1);
+            mbar_init(sbase + P::XD_EMPTY + 8 * i, KQ_EPI_WARPS);
+            mbar_init(sbase + P::ACC_FULL + 8 * i, 1);
+            mbar_init(sbase + P::ACC_EMPTY + 8 * i, KQ_EPI_WARPS);
         }
         *abort = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == K4_MMA_WARP) tmem_alloc(sbase + S::SLOT, 512);
+    if (warp == KQ_MMA_WARP) tmem_alloc(sbase + P::SLOT, 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(smem + S::SLOT);
+    const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(smem + P::SLOT);
 
-    if (warp == K4_TMA_WARP) {
+    // tile -> matrix, first row, first token; tokens change fastest, so that CTAs side by side read the same weights
+    auto locate = [&](uint32_t tile, uint32_t &row0, uint32_t &tok0) -> uint32_t {
+        const uint32_t rt = tile / a.tok_tiles;
+        tok0 = (tile - rt * a.tok_tiles) * N;
+        const uint32_t si = rt < a.tiles[0] ? 0u : rt < a.tiles[1] ? 1u : 2u;
+        row0 = (rt - (si ? a.tiles[si - 1] : 0u)) * TC_M;
+        return si;
+    };
+
+    if (warp == KQ_TMA_WARP) {
         if (lane == 0) {
-            for (uint32_t u = 0; u < n_visits; ++u) {
-                const uint32_t slot = u % IN_STAGES, s = u % nb;
-                const bool min_sweep = GEMM && u < nb;
-                if (u >= IN_STAGES && !mbar_wait(sbase + S::IN_EMPTY + 8 * slot, ((u / IN_STAGES) & 1u) ^ 1u, abort)) break;
-                const uint32_t full = sbase + S::IN_FULL + 8 * slot;
-                mbar_expect_tx(full, (min_sweep ? TC_M * 16u : K4_RAW_BYTES) + S::B_BYTES);
-                if (min_sweep) tma_load_2d(sbase + S::RAW + slot * K4_RAW_BYTES, &tm_hdr, (int32_t)(s * 144), (int32_t)row0, full);  // the 16-byte headers
-                else tma_load_2d(sbase + S::RAW + slot * K4_RAW_BYTES, &tm_raw, (int32_t)(s * 144), (int32_t)row0, full);
-                tma_load_2d(sbase + S::B + slot * S::B_BYTES, &tm_x, (int32_t)(s * 256), (int32_t)tok0, full);
-                tma_load_2d(sbase + S::B + slot * S::B_BYTES + N * 128, &tm_x, (int32_t)(s * 256 + 128), (int32_t)tok0, full);
-            }
-        }
-    } else if (warp == K4_MMA_WARP) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_i8(0, 1, N);  // unsigned planes x signed activations
+            Ring<P::RAW_STAGES> raw;
+            Ring<P::B_STAGES> bs;
+            uint32_t it = 0;
             bool ok = true;
-            for (uint32_t u = 0; u < n_visits && ok; ++u) {
-                const uint32_t slot = u % IN_STAGES, buf = u % NBUF, np = n_planes(u);
-                for (uint32_t h = 0; h < 2; ++h) {
-                    const uint32_t v = 2 * u + h, ps = v & 1u;
-                    if (!(ok = mbar_wait(sbase + S::PL_FULL + 8 * ps, (v / 2) & 1u, abort))) break;
-                    if (h == 0) {
-                        if (!(ok = mbar_wait(sbase + S::IN_FULL + 8 * slot, (u / IN_STAGES) & 1u, abort))) break;
-                        if (u >= NBUF && !(ok = mbar_wait(sbase + S::ACC_EMPTY + 8 * buf, ((u / NBUF) & 1u) ^ 1u, abort))) break;
-                    }
-                    tc_fence_after();
-                    const uint64_t db = umma_desc_sw128(sbase + S::B + slot * S::B_BYTES + h * N * 128);
-                    for (uint32_t p = 0; p < np; ++p) {
-                        const uint64_t da = umma_desc_sw128(sbase + S::PLANES + (ps * 3 + p) * K4_PLANE_BYTES);
+            auto load_b = [&](const CUtensorMap *tm, uint32_t x, uint32_t tok0, uint32_t sums) {
+                if (bs.round && !mbar_wait(sbase + P::B_EMPTY + 8 * bs.at, bs.empty_parity(), abort)) return false;
+                const uint32_t full = sbase + P::B_FULL + 8 * bs.at, dst = sbase + P::B + bs.at * P::B_STAGE;
+                mbar_expect_tx(full, P::B_STAGE);
 #pragma unroll
-                        for (uint32_t k = 0; k < 4; ++k) umma_i8(tmem + buf * ACC_STRIDE + p * N, da + 2 * k, db + 2 * k, idesc, (h | k) ? 1u : 0u);
-                    }
-                    umma_commit(sbase + S::PL_EMPTY + 8 * ps);
-                    if (h == 1) {
-                        umma_commit(sbase + S::IN_EMPTY + 8 * slot);
-                        umma_commit(sbase + S::ACC_FULL + 8 * buf);
-                    }
+                for (uint32_t i = 0; i < 4; ++i) tma_load_2d(dst + i * N * 128, tm, (int32_t)(x + 64 * i), (int32_t)tok0, full);
+                if (!GEMM) tma_load_2d(dst + N * 512, &maps.bs, (int32_t)sums, (int32_t)tok0, full);
+                bs.next();
+                return true;
+            };
+            for (uint32_t tile = blockIdx.x; tile < a.n_tiles && ok; tile += gridDim.x, ++it) {
+                uint32_t row0, tok0;
+                const uint32_t si = locate(tile, row0, tok0);
+                {   // token scales of the tile
+                    const uint32_t xs = it % a.n_xd, xr = it / a.n_xd;
+                    if (xr && !(ok = mbar_wait(sbase + P::XD_EMPTY + 8 * xs, (xr & 1u) ^ 1u, abort))) break;
+                    mbar_expect_tx(sbase + P::XD_FULL + 8 * xs, nb * N * 4);
+                    tma_load_2d(sbase + P::XD + xs * P::xd_bytes(nb), &maps.xd, (int32_t)tok0, 0, sbase + P::XD_FULL + 8 * xs);
+                }
+                for (uint32_t j = 0; j < n_min && ok; ++j) ok = load_b(&maps.bs, j * 256, tok0, 0);
+                for (uint32_t s = 0; s < nb && ok; ++s) {
+                    if (raw.round && !(ok = mbar_wait(sbase + P::RAW_EMPTY + 8 * raw.at, raw.empty_parity(), abort))) break;
+                    mbar_expect_tx(sbase + P::RAW_FULL + 8 * raw.at, KQ_RAW_BYTES);
+                    tma_load_2d(sbase + P::RAW + raw.at * KQ_RAW_BYTES, &maps.raw[si], (int32_t)(s * 144), (int32_t)row0, sbase + P::RAW_FULL + 8 * raw.at);
+                    raw.next();
+                    ok = load_b(&maps.x, s * 256, tok0, (s & ~3u) * 16);
                 }
             }
         }
-    } else if (warp >= TC_EPI_WARPS) {
-        // ---- expanders: thread = one row of the half super-block in flight (two runs of 64 elements)
-        const uint32_t r = threadIdx.x - TC_EPI_WARPS * 32;
-        const uint32_t swz = r & 7u, row_off = (r >> 3) * 1024 + swz * 128;
+    } else if (warp == KQ_MMA_WARP) {
+        constexpr uint32_t idesc = umma_idesc_f16(N), BOX = N * 128 / 16;
+        Ring<P::B_STAGES> bs;
+        Ring<2> ab, ac;
         bool ok = true;
-        for (uint32_t u = 0; u < n_visits && ok; ++u) {
-            const uint32_t slot = u % IN_STAGES, s = u % nb;
-            const bool min_sweep = GEMM && u < nb, main_sweep = GEMM && u >= nb;
-            if (!(ok = mbar_wait(sbase + S::IN_FULL + 8 * slot, (u / IN_STAGES) & 1u, abort))) break;
-            const uint8_t *raw = smem + S::RAW + slot * K4_RAW_BYTES + r * (min_sweep ? 16u : 144u);
-            const uint4 hd = *reinterpret_cast<const uint4 *>(raw);
-            reinterpret_cast<uint32_t *>(smem + S::DD)[(u % K4_RING) * TC_M + r] = hd.x;
-            if (r < (uint32_t)N) {
-                const uint32_t tok = tok0 + r;
-                reinterpret_cast<float *>(smem + S::XD)[(u % K4_RING) * N + r] = tok < a.n_tokens ? __ldg(a.act_d + (uint64_t)tok * a.act_d_pitch + s) : 0.0f;
-            }
-            // the eight 6-bit scales and mins (engine/quant.rs:653-662) as bytes of two words each
-            const uint32_t scl = hd.y & 0x3f3f3f3fu, ml = hd.z & 0x3f3f3f3fu;
-            const uint32_t sch = (hd.w & 0x0f0f0f0fu) | ((hd.y >> 2) & 0x30303030u), mh = ((hd.w >> 4) & 0x0f0f0f0fu) | ((hd.z >> 2) & 0x30303030u);
-            for (uint32_t h = 0; h < 2; ++h) {
-                const uint32_t v = 2 * u + h, ps = v & 1u;
-                if (v >= 2 && !(ok = mbar_wait(sbase + S::PL_EMPTY + 8 * ps, ((v / 2) & 1u) ^ 1u, abort))) break;
-                uint8_t *pl = smem + S::PLANES + ps * 3 * K4_PLANE_BYTES + row_off;
-#pragma unroll
-                for (uint32_t gl = 0; gl < 2; ++gl) {
-                    const uint32_t g = 2 * h + gl;  // 64 elements 64 g .. of the super-block: sub-blocks 2g (low nibbles), 2g + 1 (high)
-                    const uint32_t scw = h == 0 ? scl : sch, mw = h == 0 ? ml : mh, sh = 16 * gl;
-                    const uint32_t sa = (scw >> sh) & 0xffu, sb = (scw >> (sh + 8)) & 0xffu, ma = (mw >> sh) & 0xffu, mb = (mw >> (sh + 8)) & 0xffu;
-                    // 16-byte chunks 4 gl .. 4 gl + 3 of the row's 128 bytes, swizzled: low-nibble sub-block in the first two, high in the last two
-                    const uint32_t c0 = ((4 * gl + 0) ^ swz) * 16, c1 = ((4 * gl + 1) ^ swz) * 16, c2 = ((4 * gl + 2) ^ swz) * 16, c3 = ((4 * gl + 3) ^ swz) * 16;
-                    if (!min_sweep) {
-                        const uint4 qa = *reinterpret_cast<const uint4 *>(raw + 16 + 32 * g), qb = *reinterpret_cast<const uint4 *>(raw + 32 + 32 * g);
-                        const uint32_t M = 0x0f0f0f0fu;
-                        const uint32_t la[8] = {qa.x & M, qa.y & M, qa.z & M, qa.w & M, qb.x & M, qb.y & M, qb.z & M, qb.w & M};
-                        const uint32_t ha[8] = {(qa.x >> 4) & M, (qa.y >> 4) & M, (qa.z >> 4) & M, (qa.w >> 4) & M, (qb.x >> 4) & M, (qb.y >> 4) & M, (qb.z >> 4) & M, (qb.w >> 4) & M};
-                        const uint32_t sal = sa & 7u, sah = sa >> 3, sbl = sb & 7u, sbh = sb >> 3;
-                        uint8_t *plo = pl, *phi = pl + K4_PLANE_BYTES;
-                        // four codes (each <= 15) times a digit (<= 7) in one multiply: no byte reaches 256
-                        *reinterpret_cast<uint4 *>(plo + c0) = make_uint4(la[0] * sal, la[1] * sal, la[2] * sal, la[3] * sal);
-                        *reinterpret_cast<uint4 *>(plo + c1) = make_uint4(la[4] * sal, la[5] * sal, la[6] * sal, la[7] * sal);
-                        *reinterpret_cast<uint4 *>(plo + c2) = make_uint4(ha[0] * sbl, ha[1] * sbl, ha[2] * sbl, ha[3] * sbl);
-                        *reinterpret_cast<uint4 *>(plo + c3) = make_uint4(ha[4] * sbl, ha[5] * sbl, ha[6] * sbl, ha[7] * sbl);
-                        *reinterpret_cast<uint4 *>(phi + c0) = make_uint4(la[0] * sah, la[1] * sah, la[2] * sah, la[3] * sah);
-                        *reinterpret_cast<uint4 *>(phi + c1) = make_uint4(la[4] * sah, la[5] * sah, la[6] * sah, la[7] * sah);
-                        *reinterpret_cast<uint4 *>(phi + c2) = make_uint4(ha[0] * sbh, ha[1] * sbh, ha[2] * sbh, ha[3] * sbh);
-                        *reinterpret_cast<uint4 *>(phi + c3) = make_uint4(ha[4] * sbh, ha[5] * sbh, ha[6] * sbh, ha[7] * sbh);
-                    }
-                    if (!main_sweep) {
-                        uint8_t *pm = pl + (GEMM ? 0u : 2u * K4_PLANE_BYTES);
-                        const uint32_t wa = ma * 0x01010101u, wb = mb * 0x01010101u;
-                        *reinterpret_cast<uint4 *>(pm + c0) = make_uint4(wa, wa, wa, wa);
-                        *reinterpret_cast<uint4 *>(pm + c1) = make_uint4(wa, wa, wa, wa);
-                        *reinterpret_cast<uint4 *>(pm + c2) = make_uint4(wb, wb, wb, wb);
-                        *reinterpret_cast<uint4 *>(pm + c3) = make_uint4(wb, wb, wb, wb);
-                    }
+        auto wait_operands = [&] {
+            const uint32_t b = sbase + P::B_FULL + 8 * bs.at, x = sbase + P::A_FULL + 8 * ab.at;
+            if (__all_sync(0xffffffffu, mbar_try2(x, ab.full_parity(), b, bs.full_parity()))) return true;
+            return mbar_wait_warp(b, bs.full_parity(), abort) && mbar_wait_warp(x, ab.full_parity(), abort);
+        };
+        auto wait_slot = [&] { return !ac.round || __all_sync(0xffffffffu, mbar_wait_ready(sbase + P::ACC_EMPTY + 8 * ac.at, ac.empty_parity(), abort)); };
+        auto stage_done = [&] {
+            umma_commit_warp(sbase + P::A_EMPTY + 8 * ab.at);
+            umma_commit_warp(sbase + P::B_EMPTY + 8 * bs.at);
+            ab.next();
+            bs.next();
+        };
+        for (uint32_t tile = blockIdx.x; tile < a.n_tiles && ok; tile += gridDim.x) {
+            for (uint32_t j = 0; j < n_min && ok; ++j) {  // sixteen super-blocks of mins
+                if (!(ok = wait_operands())) break;
+                const uint64_t db = umma_desc_sw128(sbase + P::B + bs.at * P::B_STAGE);
+                const uint32_t ta = tmem + P::A_COL + ab.at * KQ_A_COLS;
+                for (uint32_t i = 0; i < 16 && 16 * j + i < nb; ++i) {
+                    if (!(ok = wait_slot())) break;
+                    tc_fence_after();
+                    const uint32_t td = tmem + ac.at * P::SLOT_COLS;
+                    const uint64_t d = db + (i >> 2) * BOX + (i & 3u) * 2;
+                    umma_bf16_ta_warp(td, ta + 8 * i, d, idesc, 0u);
+                    umma_commit_warp(sbase + P::ACC_FULL + 8 * ac.at);
+                    ac.next();
                 }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads these planes through the async proxy
-                __syncwarp();
-                if (lane == 0) mbar_arrive(sbase + S::PL_FULL + 8 * ps);
+                if (ok) stage_done();
+            }
+            for (uint32_t s = 0; s < nb && ok; ++s) {
+                const uint32_t ta = tmem + P::A_COL + ab.at * KQ_A_COLS;
+                const uint64_t db = umma_desc_sw128(sbase + P::B + bs.at * P::B_STAGE);
+                if (!(ok = wait_slot() && wait_operands())) break;
+                tc_fence_after();
+                uint32_t td = tmem + ac.at * P::SLOT_COLS;
+                umma_f16_ta_8(td, ta, db, BOX, idesc, 0u);
+                if (TWO) {  // the halves' sums apart
+                    umma_commit_warp(sbase + P::ACC_FULL + 8 * ac.at);
+                    ac.next();
+                    if (!(ok = wait_slot())) break;
+                    tc_fence_after();
+                    td = tmem + ac.at * P::SLOT_COLS;
+                }
+                umma_f16_ta_8(td, ta + 64, db + 2 * BOX, BOX, idesc, TWO ? 0u : 1u);
+                if (!GEMM) umma_bf16_ta_warp(td + N, tmem + P::MIN_COL + 8 * ab.at, db + 4 * BOX + (s & 3u) * 2, idesc, 0u);
+                umma_commit_warp(sbase + P::ACC_FULL + 8 * ac.at);
+                stage_done();
+                ac.next();
+            }
+        }
+    } else if (warp >= KQ_EPI_WARPS) {
+        // ---- expanders: thread = half a super-block of one row
+        const uint32_t quad = warp & 3u, h = (warp >> 2) & 1u, r = quad * 32 + lane;
+        const uint32_t ta = tmem + ((quad * 32) << 16) + P::A_COL;
+        Ring<P::RAW_STAGES> raw;
+        Ring<2> ab;
+        bool ok = true;
+        auto wait_a = [&] { return !ab.round || mbar_wait_ready(sbase + P::A_EMPTY + 8 * ab.at, ab.empty_parity(), abort); };
+        auto store = [&](uint32_t (&w)[64]) {
+            const uint32_t to = ta + ab.at * KQ_A_COLS + 64 * h;
+            tmem_st32(to, *reinterpret_cast<uint32_t(*)[32]>(w));
+            tmem_st32(to + 32, *reinterpret_cast<uint32_t(*)[32]>(w + 32));
+        };
+        auto done_a = [&] {
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(sbase + P::A_FULL + 8 * ab.at);
+            ab.next();
+        };
+        for (uint32_t tile = blockIdx.x; tile < a.n_tiles && ok; tile += gridDim.x) {
+            uint32_t row0, tok0;
+            const GemvSegment &seg = a.seg[locate(tile, row0, tok0)];
+            const uint8_t *wrow = seg.w.data + (uint64_t)min(row0 + r, seg.w.out_dim - 1) * seg.w.row_stride;
+            for (uint32_t j = 0; j < n_min; ++j) {
+                uint32_t w[64];
+#pragma unroll
+                for (uint32_t i = 0; i < 8; ++i) {
+                    const uint4 hd = __ldg(reinterpret_cast<const uint4 *>(wrow + (uint64_t)min(16 * j + 8 * h + i, nb - 1) * 144));
+                    kq_mins(hd, w + 8 * i);
+                }
+                if (!(ok = wait_a())) break;
+                tc_fence_after();
+                store(w);
+                done_a();
             }
             if (!ok) break;
-            __syncwarp();
-            if (lane == 0) mbar_arrive(sbase + S::IN_EMPTY + 8 * slot);  // this warp is done with the blocks of the visit
+            for (uint32_t s = 0; s < nb; ++s, raw.next()) {
+                if (!(ok = mbar_wait_ready(sbase + P::RAW_FULL + 8 * raw.at, raw.full_parity(), abort))) break;
+                const uint8_t *blk = smem + P::RAW + raw.at * KQ_RAW_BYTES + r * 144u;
+                const uint4 hd = *reinterpret_cast<const uint4 *>(blk);
+                // the half's four 6-bit scales (engine/quant.rs:653-662) as bytes of a word, then each twice as f16
+                const uint32_t scw = h == 0 ? hd.y & 0x3f3f3f3fu : (hd.w & 0x0f0f0f0fu) | ((hd.y >> 2) & 0x30303030u);
+                uint32_t out[64];
+#pragma unroll
+                for (uint32_t g = 0; g < 2; ++g) {  // 64 elements: 32 low nibbles, 32 high ones
+                    const uint4 qa = *reinterpret_cast<const uint4 *>(blk + 16 + 64 * h + 32 * g), qb = *reinterpret_cast<const uint4 *>(blk + 32 + 64 * h + 32 * g);
+                    const uint32_t sa = h2_sub(__byte_perm(scw, 0x64646464u, g ? 0x4242 : 0x4040), H2_1024), sb = h2_sub(__byte_perm(scw, 0x64646464u, g ? 0x4343 : 0x4141), H2_1024);
+                    const uint32_t oa = h2_mul(sa, H2_M1024), sb16 = h2_mul(sb, H2_16TH), ob = h2_mul(sb, H2_M64);
+                    const uint32_t w[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {  // 1024 + code and 1024 + 16 code as f16 mantissas; times the scale, less 1024 times it: exact
+                        const uint32_t v = w[i] >> 8;
+                        out[32 * g + 2 * i] = h2_fma((w[i] & 0x000f000fu) | H2_1024, sa, oa);
+                        out[32 * g + 2 * i + 1] = h2_fma((v & 0x000f000fu) | H2_1024, sa, oa);
+                        out[32 * g + 16 + 2 * i] = h2_fma((w[i] & 0x00f000f0u) | H2_1024, sb16, ob);
+                        out[32 * g + 16 + 2 * i + 1] = h2_fma((v & 0x00f000f0u) | H2_1024, sb16, ob);
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(sbase + P::RAW_EMPTY + 8 * raw.at);
+                if (!(ok = wait_a())) break;
+                tc_fence_after();
+                store(out);
+                if (!GEMM && h == 1) {
+                    uint32_t w[8];
+                    kq_mins(hd, w);
+                    tmem_st8(tmem + ((quad * 32) << 16) + P::MIN_COL + 8 * ab.at, w);
+                }
+                done_a();
+            }
         }
     } else {
         // ---- epilogue: thread = one row x N / 2 tokens
         const uint32_t quad = warp & 3u, half = warp >> 2, rl = quad * 32 + lane;
-        const uint32_t row = row0 + rl;
-        const bool row_ok = row < seg.w.out_dim;
-        float acc[TPT];
+        const uint32_t tbase = tmem + ((quad * 32) << 16) + half * TPT;
+        const uint64_t ones = a.ones;
+        Ring<2> ac;
+        uint32_t it = 0;
+        bool ok = true;
+        for (uint32_t tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x, ++it) {
+            uint32_t row0, tok0;
+            const GemvSegment &seg = a.seg[locate(tile, row0, tok0)];
+            const uint32_t row = row0 + rl;
+            const uint8_t *wrow = seg.w.data + (uint64_t)min(row, seg.w.out_dim - 1) * seg.w.row_stride;
+            const uint32_t xs = it % a.n_xd, xr = it / a.n_xd;
+            if (!(ok = mbar_wait(sbase + P::XD_FULL + 8 * xs, xr & 1u, abort))) break;
+            const float *xd = reinterpret_cast<const float *>(smem + P::XD + xs * P::xd_bytes(nb)) + half * TPT;
+            uint64_t acc[TPT / 2];
 #pragma unroll
-        for (int t = 0; t < TPT; ++t) acc[t] = 0.0f;
-        for (uint32_t u = 0; u < n_visits; ++u) {
-            const uint32_t buf = u % NBUF, ring = u % K4_RING;
-            const bool min_sweep = GEMM && u < nb;
-            if (!mbar_wait(sbase + S::ACC_FULL + 8 * buf, (u / NBUF) & 1u, abort)) break;
-            tc_fence_after();
-            const uint32_t dw = reinterpret_cast<const uint32_t *>(smem + S::DD)[ring * TC_M + rl];
-            const float d = f16_bits_to_f32(dw & 0xffffu), dmin = f16_bits_to_f32(dw >> 16);
-            const float *xd = reinterpret_cast<const float *>(smem + S::XD) + ring * N + half * TPT;
-            const uint32_t tbase = tmem + ((quad * 32) << 16) + buf * ACC_STRIDE + half * TPT;
+            for (int t = 0; t < TPT / 2; ++t) acc[t] = 0ull;
+            auto header = [&](uint32_t s) { return __ldg(reinterpret_cast<const uint32_t *>(wrow + (uint64_t)min(s, nb - 1) * 144)); };  // d | dmin << 16
+            uint32_t dw0 = header(0), dw1 = header(1);
+            if (GEMM) {
+                for (uint32_t s = 0; s < nb; ++s) {
+                    const uint32_t dw2 = header(s + 2);
+                    if (!(ok = mbar_wait_ready(sbase + P::ACC_FULL + 8 * ac.at, ac.full_parity(), abort))) break;
+                    tc_fence_after();
+                    const uint64_t dmin2 = f2_both(-f16_bits_to_f32(dw0 >> 16));
+                    const float4 *ad4 = reinterpret_cast<const float4 *>(xd + s * N);
 #pragma unroll
-            for (int c = 0; c < TPT / 16; ++c) {  // 16 tokens at a time
-                uint32_t p0[16], p1[16], p2[16];
-                tmem_ld16(tbase + c * 16, p0);
-                if (!GEMM || !min_sweep) tmem_ld16(tbase + N + c * 16, p1);
-                if (!GEMM) tmem_ld16(tbase + 2 * N + c * 16, p2);
-                tmem_ld_wait();
+                    for (int c = 0; c < TPT / CH; ++c) {
+                        uint32_t p[CH];
+                        tmem_ldn<CH>(tbase + ac.at * P::SLOT_COLS + c * CH, p);
+                        tmem_ld_wait();
 #pragma unroll
-                for (int t = 0; t < 16; ++t) {
-                    const float ad = xd[c * 16 + t];
-                    float &o = acc[c * 16 + t];
-                    if (!GEMM) {
-                        const int isum = (int)(p1[t] << 3) + (int)p0[t], imin = (int)p2[t];
-                        o = __fadd_rn(o, __fmul_rn(ad, __fsub_rn(__fmul_rn(d, (float)isum), __fmul_rn(dmin, (float)imin))));
-                    } else if (min_sweep) {
-                        o = __fsub_rn(o, __fmul_rn(__fmul_rn(ad, dmin), (float)(int)p0[t]));
-                    } else {
-                        const int isum = (int)(p1[t] << 3) + (int)p0[t];
-                        o = __fadd_rn(o, __fmul_rn(ad, __fmul_rn(d, (float)isum)));
+                        for (int t = 0; t < CH / 4; ++t) {
+                            const float4 v = ad4[c * (CH / 4) + t];
+                            const uint64_t ad[2] = {f2_pack(v.x, v.y), f2_pack(v.z, v.w)};
+#pragma unroll
+                            for (int k = 0; k < 2; ++k) {
+                                uint64_t &o = acc[c * (CH / 2) + 2 * t + k];
+                                o = f2_add(f2_mul(f2_mul(ad[k], dmin2), f2_pack(p[4 * t + 2 * k], p[4 * t + 2 * k + 1])), o, ones);  // x - y = x + (-y), the sign taken with dmin
+                            }
+                        }
                     }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(sbase + P::ACC_EMPTY + 8 * ac.at);
+                    ac.next();
+                    dw0 = dw1;
+                    dw1 = dw2;
                 }
+                if (!ok) break;
+                dw0 = header(0);
+                dw1 = header(1);
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(sbase + S::ACC_EMPTY + 8 * buf);
-        }
-        if (!*abort && row_ok) {
+            auto sweep = [&] {
+                for (uint32_t s = 0; s < nb; ++s) {
+                    const uint32_t dw2 = header(s + 2);
+                    const uint64_t d2 = f2_both(f16_bits_to_f32(dw0 & 0xffffu)), dmin2 = f2_both(-f16_bits_to_f32(dw0 >> 16));
+                    const uint32_t first = ac.at;
+                    if (!mbar_wait_ready(sbase + P::ACC_FULL + 8 * ac.at, ac.full_parity(), abort)) return false;
+                    if (TWO) {
+                        ac.next();
+                        if (!mbar_wait_ready(sbase + P::ACC_FULL + 8 * ac.at, ac.full_parity(), abort)) return false;
+                    }
+                    tc_fence_after();
+                    const float4 *ad4 = reinterpret_cast<const float4 *>(xd + s * N);
+                    const uint32_t tslot = tbase + ac.at * P::SLOT_COLS;
 #pragma unroll
-            for (int t = 0; t < TPT; ++t) {
-                const uint32_t tok = tok0 + half * TPT + t;
-                if (tok < a.n_tokens) {
-                    const uint64_t o = (uint64_t)tok * seg.y_stride + row;
-                    float v = acc[t];
-                    if (seg.epilogue == EPI_ADD_RESIDUAL) v = __fadd_rn(seg.residual[o], v);
-                    seg.y[o] = v;
+                    for (int c = 0; c < TPT / CH; ++c) {
+                        uint32_t p0[CH], p1[CH], p2[CH];
+                        tmem_ldn<CH>(tslot + c * CH, p0);
+                        if (TWO) tmem_ldn<CH>(tbase + first * P::SLOT_COLS + c * CH, p1);
+                        if (!GEMM) tmem_ldn<CH>(tslot + N + c * CH, p2);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int t = 0; t < CH / 4; ++t) {
+                            const float4 v = ad4[c * (CH / 4) + t];
+                            const uint64_t ad[2] = {f2_pack(v.x, v.y), f2_pack(v.z, v.w)};
+#pragma unroll
+                            for (int k = 0; k < 2; ++k) {
+                                const int i = 4 * t + 2 * k;
+                                uint64_t &o = acc[c * (CH / 2) + 2 * t + k];
+                                uint64_t m = f2_pack(p0[i], p0[i + 1]);
+                                if (TWO) m = f2_add(m, f2_pack(p1[i], p1[i + 1]), ones);  // both are whole numbers: their rounded sum is (float)isum
+                                m = f2_mul(d2, m);
+                                if (!GEMM) m = f2_add(f2_mul(dmin2, f2_pack(p2[i], p2[i + 1])), m, ones);
+                                o = f2_add(f2_mul(ad[k], m), o, ones);
+                            }
+                        }
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(sbase + P::ACC_EMPTY + 8 * ac.at);
+                        if (TWO) mbar_arrive(sbase + P::ACC_EMPTY + 8 * first);
+                    }
+                    ac.next();
+                    dw0 = dw1;
+                    dw1 = dw2;
+                }
+                return true;
+            };
+            ok = sweep();
+            if (!ok) break;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(sbase + P::XD_EMPTY + 8 * xs);
+            if (row < seg.w.out_dim && (TWO || !__ldg(seg.w.wide + row))) {  // (wide rows are left to the kernel that follows)
+                const uint32_t t0 = tok0 + half * TPT, n = a.n_tokens > t0 ? min((uint32_t)TPT, a.n_tokens - t0) : 0u;
+                float *y = seg.y + (uint64_t)t0 * seg.y_stride + row;
+                const float *res = seg.epilogue == EPI_ADD_RESIDUAL ? seg.residual + (uint64_t)t0 * seg.y_stride + row : nullptr;
+#pragma unroll
+                for (int c = 0; c < TPT; c += 8) {
+                    float v[8];
+#pragma unroll
+                    for (int t = 0; t < 8; ++t) v[t] = res && c + t < (int)n ? res[(uint64_t)(c + t) * seg.y_stride] : 0.0f;
+#pragma unroll
+                    for (int t = 0; t < 8; ++t) {
+                        const float o = t & 1 ? f2_hi(acc[(c + t) / 2]) : f2_lo(acc[(c + t) / 2]);
+                        if (c + t < (int)n) y[(uint64_t)(c + t) * seg.y_stride] = res ? __fadd_rn(v[t], o) : o;
+                    }
                 }
             }
         }
     }
-    if (*abort) {
+    pdl_wait();  // started beside the kernel of the wide rows (launch_q4k_instance), this one does not end before it
+    if (*abort) {  // let copies that are still in flight land before the shared memory goes away
         for (int i = 0; i < 200; ++i) __nanosleep(1000);
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == K4_MMA_WARP) tmem_dealloc(tmem, 512);
+    if (warp == KQ_MMA_WARP) tmem_dealloc(tmem, 512);
 }
 
 }  // namespace
@@ -438,13 +636,7 @@ bool gemm_tc5_supported(const GemvArgs &a) {
     if (type == TYPE_Q8_0) {
         if (in_dim % 128 || a.act.dim_cap % 128) return false;
     } else if (type == TYPE_Q4_K) {
-        if (in_dim % 256 || a.act.dim_cap % 16) return false;
-        // A CTA owns 128 rows x 64 or 128 tokens and walks the whole row (the fp32 order forbids splitting K), so a small
-        // matrix at a small batch gives too few CTAs: the 64-row mma.sync tiles (gemm_mma.cu) fill the GPU better there.
-        uint32_t ctas = 0;
-        const uint32_t tok_tile = a.n_tokens > 64 ? 128 : 64;
-        for (int s = 0; s < a.n_seg; ++s) ctas += ((a.seg[s].w.out_dim + TC_M - 1) / TC_M) * ((a.n_tokens + tok_tile - 1) / tok_tile);
-        if (ctas < 96) return false;
+        if (in_dim % 256 || in_dim / 256 > 256 || !a.act.h || a.act.dim_cap % 256) return false;
     } else {
         return false;  // Q6_K stays on the mma.sync tiles (gemm_mma.cu)
     }
@@ -453,45 +645,112 @@ bool gemm_tc5_supported(const GemvArgs &a) {
     return true;
 }
 
-template <bool GEMM, int N>
+template <bool GEMM, bool TWO, int N>
 static bool launch_q4k_instance(const GemvArgs &a, int sm_count, cudaStream_t st) {
+    using P = KqPlan<GEMM, N>;
     static PerDeviceOnce once;
-    if (once.run([] { return cudaFuncSetAttribute(gemm_tc5_q4k_kernel<GEMM, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, K4Smem<N>::ALLOC); }) != cudaSuccess) return false;
+    if (once.run([] { return cudaFuncSetAttribute(gemm_tc5_q4k_kernel<GEMM, TWO, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); }) != cudaSuccess) return false;
     const uint32_t in_dim = a.seg[0].w.in_dim, nb = in_dim / 256;
-    CUtensorMap tm_x;
-    if (!make_map_2d(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.act.q, in_dim, a.n_tokens, a.act.dim_cap, 128, N, CU_TENSOR_MAP_SWIZZLE_128B)) return false;
-    auto maps = [&](const GemvSegment &g, CUtensorMap *raw, CUtensorMap *hdr) {
-        return make_map_2d(raw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, g.w.data, (uint64_t)nb * 144, g.w.out_dim, g.w.row_stride, 144, TC_M, CU_TENSOR_MAP_SWIZZLE_NONE) &&
-               make_map_2d(hdr, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, g.w.data, (uint64_t)nb * 144, g.w.out_dim, g.w.row_stride, 16, TC_M, CU_TENSOR_MAP_SWIZZLE_NONE);
-    };
-    const uint32_t tok_tiles = (a.n_tokens + N - 1) / N, sms = (uint32_t)std::max(1, sm_count);
-    auto tiles = [&](int s) { return (a.seg[s].w.out_dim + TC_M - 1) / TC_M; };
-    auto waves = [&](uint32_t ctas) { return (ctas + sms - 1) / sms; };
-    for (int s = 0; s < a.n_seg; ++s) {
-        // pair this matrix with the next one when one launch takes fewer waves than two
-        const bool pair = s + 1 < a.n_seg && waves((tiles(s) + tiles(s + 1)) * tok_tiles) < waves(tiles(s) * tok_tiles) + waves(tiles(s + 1) * tok_tiles);
-        CUtensorMap raw0, hdr0, raw1, hdr1;
-        if (!maps(a.seg[s], &raw0, &hdr0) || !maps(a.seg[pair ? s + 1 : s], &raw1, &hdr1)) return false;
-        TcK4Args k{};
-        k.seg = a.seg[s];
-        k.seg2 = a.seg[pair ? s + 1 : s];
-        k.tiles0 = tiles(s);
-        k.act_d = a.act.d;
-        k.act_d_pitch = a.act.dim_cap / 256;
-        k.n_tokens = a.n_tokens;
-        k.nb = nb;
-        const dim3 grid(tiles(s) + (pair ? tiles(s + 1) : 0u), tok_tiles);
-        gemm_tc5_q4k_kernel<GEMM, N><<<grid, K4_THREADS, K4Smem<N>::ALLOC, st>>>(raw0, hdr0, raw1, hdr1, tm_x, k);
-        g_tc5_launched.store(true, std::memory_order_relaxed);
-        if (pair) ++s;
+    KqArgs k{};
+    KqMaps m;
+    k.n_xd = P::bytes(nb, 2) <= 227 * 1024 ? 2 : 1;
+    if (P::bytes(nb, k.n_xd) > 227 * 1024) return false;
+    if (!make_map_2d(&m.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.act.h, in_dim, a.n_tokens, (uint64_t)a.act.dim_cap * 2, 64, N, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !make_map_2d(&m.bs, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.act.hs, in_dim / 16, a.n_tokens, a.act.dim_cap / 16 * 2, 64, N, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !make_map_2d(&m.xd, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a.act.dt, a.n_tokens, nb, (uint64_t)a.act.dt_pitch * 4, N, nb, CU_TENSOR_MAP_SWIZZLE_NONE))
+        return false;
+    uint32_t row_tiles = 0;
+    for (int s = 0; s < 3; ++s) {
+        const int used = std::min(s, a.n_seg - 1);
+        k.seg[s] = a.seg[used];
+        const DevWeight &w = k.seg[s].w;
+        if (!make_map_2d(&m.raw[s], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w.data, (uint64_t)nb * 144, w.out_dim, w.row_stride, 144, TC_M, CU_TENSOR_MAP_SWIZZLE_NONE)) return false;
+        if (s < a.n_seg) row_tiles += (w.out_dim + TC_M - 1) / TC_M;
+        k.tiles[s] = row_tiles;
     }
+    k.ones = F2_ONES;
+    k.n_tokens = a.n_tokens;
+    k.nb = nb;
+    k.tok_tiles = (a.n_tokens + N - 1) / N;
+    k.n_tiles = row_tiles * k.tok_tiles;
+    // Wide rows first, in a kernel that lets this one start beside it: neither reads what the other writes, and both read what was complete
+    // before the first of them started.
+    bool beside = false;
+    for (int s = 0; s < a.n_seg && !TWO; ++s) {
+        if (!a.seg[s].w.n_wide) continue;
+        if (!launch_gemm_few_rows(a, s, sm_count, st)) return false;
+        beside = true;
+    }
+    const uint32_t grid = std::min(k.n_tiles, (uint32_t)std::max(1, sm_count));
+    if (beside) launch_pdl(gemm_tc5_q4k_kernel<GEMM, TWO, N>, grid, KQ_THREADS, P::bytes(nb, k.n_xd), st, m, k);
+    else gemm_tc5_q4k_kernel<GEMM, TWO, N><<<grid, KQ_THREADS, P::bytes(nb, k.n_xd), st>>>(m, k);
+    g_tc5_launched.store(true, std::memory_order_relaxed);
     return true;
 }
 
+// How the product of Q4_K matrices is cut: tokens per tile, whether halves are kept apart, and about how long it takes.
+struct KqChoice {
+    uint32_t n = 0;
+    bool two = false;
+    double us = 1e30;
+};
+static KqChoice choose_q4k(const GemvArgs &a, int sm_count) {
+    KqChoice best;
+    // A few wide rows are computed apart; a matrix with one in 128 or more keeps all halves apart, which is slower for all of its rows.
+    bool wide = false;
+    for (int s = 0; s < a.n_seg; ++s) {
+        const DevWeight &w = a.seg[s].w;
+        wide = wide || w.n_wide;
+        best.two = best.two || w.n_wide > (gemm_few_rows_supported(a) ? w.out_dim / 128 : 0u);
+    }
+    uint32_t rows = 0;
+    for (int s = 0; s < a.n_seg; ++s) rows += (a.seg[s].w.out_dim + TC_M - 1) / TC_M;
+    // Microseconds that a tile takes per super-block (4096 x 14336 and 14336 x 4096, 64 to 512 tokens).  Wider tiles lose their registers.
+    struct Width {
+        uint32_t n;
+        double prefill, decode;  // 0: not built
+    };
+    for (const Width &w : {Width{96, 1.57, 0}, Width{64, 1.45, 0}, Width{48, 0, 0.95}, Width{32, 1.15, 0.88}, Width{16, 1.08, 0.83}}) {
+        const double each = a.gemm_order ? w.prefill : w.decode;
+        if (each == 0 || (best.two && w.n > (a.gemm_order ? 64u : 32u))) continue;
+        const uint32_t nb = a.seg[0].w.nb, raw = (w.n > 64 ? 3u : 4u) * KQ_RAW_BYTES, b = (w.n > 64 ? 2u : 3u) * w.n * (a.gemm_order ? 512u : 640u);
+        if (raw + b + nb * w.n * 4 + 2048 > 227 * 1024) continue;
+        const uint32_t tiles = rows * ((a.n_tokens + w.n - 1) / w.n), waves = (tiles + sm_count - 1) / sm_count;
+        const double us = 4.0 + (wide ? 3.0 : 0.0) + (best.two ? 1.3 : 1.0) * waves * nb * each;
+        if (us < best.us) best.us = us, best.n = w.n;
+    }
+    return best;
+}
+double gemm_tc5_q4k_us(const GemvArgs &a, int sm_count) { return choose_q4k(a, std::max(1, sm_count)).us; }
+
 static bool launch_q4k(const GemvArgs &a, int sm_count, cudaStream_t st) {
-    const bool wide = a.n_tokens > 64;  // 128-token tiles once there are tokens for them
-    if (a.gemm_order) return wide ? launch_q4k_instance<true, 128>(a, sm_count, st) : launch_q4k_instance<true, 64>(a, sm_count, st);
-    return wide ? launch_q4k_instance<false, 128>(a, sm_count, st) : launch_q4k_instance<false, 64>(a, sm_count, st);
+    const KqChoice c = choose_q4k(a, std::max(1, sm_count));
+    if (a.gemm_order && !c.two) {
+        switch (c.n) {
+        case 96: return launch_q4k_instance<true, false, 96>(a, sm_count, st);
+        case 64: return launch_q4k_instance<true, false, 64>(a, sm_count, st);
+        case 32: return launch_q4k_instance<true, false, 32>(a, sm_count, st);
+        case 16: return launch_q4k_instance<true, false, 16>(a, sm_count, st);
+        }
+    } else if (a.gemm_order) {
+        switch (c.n) {
+        case 64: return launch_q4k_instance<true, true, 64>(a, sm_count, st);
+        case 32: return launch_q4k_instance<true, true, 32>(a, sm_count, st);
+        case 16: return launch_q4k_instance<true, true, 16>(a, sm_count, st);
+        }
+    } else if (!c.two) {
+        switch (c.n) {
+        case 48: return launch_q4k_instance<false, false, 48>(a, sm_count, st);
+        case 32: return launch_q4k_instance<false, false, 32>(a, sm_count, st);
+        case 16: return launch_q4k_instance<false, false, 16>(a, sm_count, st);
+        }
+    } else {
+        switch (c.n) {
+        case 32: return launch_q4k_instance<false, true, 32>(a, sm_count, st);
+        case 16: return launch_q4k_instance<false, true, 16>(a, sm_count, st);
+        }
+    }
+    return false;  // a row too long for any tile
 }
 
 bool launch_gemm_tc5(const GemvArgs &a, int sm_count, cudaStream_t st) {

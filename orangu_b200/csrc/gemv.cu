@@ -439,7 +439,7 @@ size_t gemv_smem_bytes(uint32_t type, uint32_t in_dim, uint32_t tile_tokens, boo
 
 uint32_t gemv_launches(uint32_t type, uint32_t in_dim, uint32_t n_tokens, bool gemm_order) {
     if (type == TYPE_Q5_K) return 1;
-    if ((type == TYPE_Q4_K || type == TYPE_Q6_K) && n_tokens >= 9) return 1;  // the tensor-core kernel covers all tokens in one launch
+    if ((type == TYPE_Q4_K || type == TYPE_Q6_K) && n_tokens >= 2) return 1;  // the tensor-core kernels cover all tokens in one launch (wide rows apart)
     uint32_t T = 8;
     while (T > 1 && (T / 2 >= n_tokens || gemv_smem_bytes(type, in_dim, T, gemm_order) > 200 * 1024)) T /= 2;
     return (n_tokens + T - 1) / T;
@@ -452,7 +452,16 @@ void launch_gemv(const GemvArgs &a, int sm_count, cudaStream_t st) {
         return;
     }
     static const bool use_mma = [] { const char *e = getenv("OB_MMA"); return !(e && e[0] == '0' && e[1] == 0); }();
-    if (gemm_tc5_supported(a) && launch_gemm_tc5(a, sm_count, st)) return;  // many tokens: tcgen05 tiles (gemm_tc5.cu)
+    const bool tc5 = gemm_tc5_supported(a);
+    if (gemm_few_supported(a)) {
+        // A few tokens (gemm_few.cu).  Against tcgen05 tiles by what both take; Q6_K has none, and its 64-row tiles (gemm_mma.cu) overtake
+        // at 32768 x 4096 with 17 tokens (72 us against 108), at 4096 x 14336 with 33 (86 against 88).
+        uint32_t rows = 0;
+        for (int s = 0; s < a.n_seg; ++s) rows += a.seg[s].w.out_dim;
+        const bool few = tc5 ? gemm_few_us(a) < gemm_tc5_q4k_us(a, sm_count) : a.n_tokens <= 16 || (a.n_tokens <= 32 && rows <= 8192);
+        if (few && launch_gemm_few(a, sm_count, st)) return;
+    }
+    if (tc5 && launch_gemm_tc5(a, sm_count, st)) return;  // many tokens: tcgen05 tiles (gemm_tc5.cu)
     if (use_mma && gemm_mma_supported(a)) {  // many tokens: tensor-core tiles (gemm_mma.cu)
         launch_gemm_mma(a, sm_count, st);
         return;

@@ -16,6 +16,7 @@ namespace ob {
 // ---- formats.cu
 // src_type: the GGUF type of `src`; w.type is what the device holds (TYPE_Q8_0 for the per-32 symmetric source types).
 OB_QUANT void launch_repack(const uint8_t *src, uint64_t src_row_bytes, uint32_t src_type, uint32_t row0, uint32_t blk0, const DevWeight &w, cudaStream_t st);
+OB_QUANT void launch_q4k_wide(const DevWeight &w, uint8_t *wide, cudaStream_t st);  // fills DevWeight::wide, which was zero
 OB_QUANT void launch_dequant_rows(const DevWeight &w, uint32_t first_row, uint32_t n_rows, float *out, cudaStream_t st);
 OB_QUANT void launch_embed(const DevWeight &w, const uint32_t *tokens, uint32_t n_tokens, float *out, cudaStream_t st);
 
@@ -26,7 +27,13 @@ struct ActBuf {
     float *d = nullptr;      // [rows][dim/group]
     int16_t *sums = nullptr; // [rows][dim/16]
     uint32_t dim_cap = 0;    // row pitch in elements
+    // per-256 only, for the tcgen05 products of Q4_K (gemm_tc5.cu); written for ACT_H_ROWS rows or more
+    __half *h = nullptr;     // [rows][dim] the codes as f16, elements 0 2 1 3 of every four
+    __half *hs = nullptr;    // [rows][dim/16] per 256: the eight sums of 32 as lo + 64 hi, the lows (-32 .. 31), then the highs
+    float *dt = nullptr;     // [dim/256][dt_pitch] d with the rows side by side
+    uint32_t dt_pitch = 0;   // a multiple of 4
 };
+constexpr uint32_t ACT_H_ROWS = 16;
 enum ActSource { ACT_PLAIN = 0, ACT_RMSNORM = 1, ACT_SWIGLU = 2 };
 struct QuantArgs {
     const float *x;       // [n_rows][dim]   (PLAIN, RMSNORM) or gate (SWIGLU)
@@ -65,6 +72,13 @@ OB_QUANT uint32_t gemv_launches(uint32_t type, uint32_t in_dim, uint32_t n_token
 // ---- q5k.cu: Q5_K weights, one kernel for any token count and both fp32 orders
 OB_QUANT void launch_q5k(const GemvArgs &a, int sm_count, cudaStream_t st);
 
+// ---- gemm_few.cu: a few tokens (2 or more) against Q4_K or Q6_K, terms of a sum split over warps
+OB_QUANT bool gemm_few_supported(const GemvArgs &a);
+OB_QUANT bool launch_gemm_few(const GemvArgs &a, int sm_count, cudaStream_t st);
+OB_QUANT double gemm_few_us(const GemvArgs &a);  // about how long it takes
+OB_QUANT bool gemm_few_rows_supported(const GemvArgs &a);
+OB_QUANT bool launch_gemm_few_rows(const GemvArgs &a, int segment, int sm_count, cudaStream_t st);  // only the wide rows of a segment, any number of tokens
+
 // ---- gemm_mma.cu: many-token products on the tensor cores (Q4_K and Q6_K; 9 tokens or more)
 OB_QUANT bool gemm_mma_supported(const GemvArgs &a);
 OB_QUANT void launch_gemm_mma(const GemvArgs &a, int sm_count, cudaStream_t st);
@@ -72,6 +86,7 @@ OB_QUANT void launch_gemm_mma(const GemvArgs &a, int sm_count, cudaStream_t st);
 // ---- gemm_tc5.cu: many-token products on tcgen05 tensor cores with TMEM accumulators, TMA-fed (16 tokens or more)
 OB_QUANT bool gemm_tc5_supported(const GemvArgs &a);
 OB_QUANT bool launch_gemm_tc5(const GemvArgs &a, int sm_count, cudaStream_t st);  // false: a tensor map could not be made (nothing was launched)
+OB_QUANT double gemm_tc5_q4k_us(const GemvArgs &a, int sm_count);  // about how long it takes
 OB_QUANT int gemm_tc5_take_status();  // 1 when a bounded wait inside one of these kernels ran out since the last call
 
 // ---- stream_gemv.cu: fused single-token products for decode (Q4_K / Q6_K weights)

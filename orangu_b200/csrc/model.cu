@@ -53,6 +53,12 @@ int alloc_act(ob_model *m, ActPair *a, uint32_t rows, uint32_t dim) {
         if ((rc = dev_alloc(m, &b->sums, (size_t)rows * (dim / 16)))) return rc;
         b->dim_cap = dim;
     }
+    if (rows >= ACT_H_ROWS && dim % 256 == 0) {
+        a->k.dt_pitch = (rows + 3) / 4 * 4;
+        if ((rc = dev_alloc(m, &a->k.h, (size_t)rows * dim))) return rc;
+        if ((rc = dev_alloc(m, &a->k.hs, (size_t)rows * (dim / 16)))) return rc;
+        if ((rc = dev_alloc(m, &a->k.dt, (size_t)(dim / 256) * a->k.dt_pitch))) return rc;
+    }
     return OB_OK;
 }
 

@@ -26,7 +26,7 @@ struct ob_ctx {
     std::string err;
     uint64_t launches = 0;
     float last_ms = 0.0f;
-    Scratch sx, sy, sq, sd, ss, saux, saux2, saux3;
+    Scratch sx, sy, sq, sd, ss, sh, shs, sdt, saux, saux2, saux3;
 };
 
 struct ob_weight {
