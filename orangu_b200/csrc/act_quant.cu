@@ -6,7 +6,8 @@
 // Every step is an IEEE single operation, so the int8 codes and the scales equal the CPU's
 // bit for bit whenever the fp32 input does.
 //
-// One CTA per token row.  A thread owns 8 consecutive elements; a warp owns one 256-block.
+// One CTA per token row, or several where nothing needs the whole row and rows are few.  A thread owns 8 consecutive elements; a warp
+// owns one 256-block.
 #include "common.cuh"
 #include "kernels.h"
 #include "seqsum.cuh"
@@ -59,7 +60,7 @@ __global__ void __launch_bounds__(QT) quantize_kernel(QuantArgs a) {
     }
 
     const uint32_t n_chunks = dim / 8;
-    for (uint32_t c = threadIdx.x; c < ((n_chunks + 31) & ~31u); c += QT) {
+    for (uint32_t c = blockIdx.y * QT + threadIdx.x; c < ((n_chunks + 31) & ~31u); c += gridDim.y * QT) {
         const bool live = c < n_chunks;
         float v[8];
         if (live) {
@@ -150,8 +151,12 @@ void launch_quantize(int source, const QuantArgs &args, cudaStream_t st) {
     QuantArgs a = args;
     if (a.n_rows == 0) return;
     if (a.n_rows < ACT_H_ROWS) a.k.h = nullptr;
+    // A row of 14336 is four passes of a CTA, and the exponentials of a SwiGLU are 8 us of them one after the other: few rows are shared out
+    // (9.8 us for 8 rows by a CTA each), until CTAs are two to an SM or so.
+    const uint32_t passes = (a.dim + QT * 8 - 1) / (QT * 8);
+    const dim3 grid(a.n_rows, a.n_rows * passes <= 296 ? passes : 1);
     switch (source) {
-    case ACT_PLAIN: quantize_kernel<ACT_PLAIN><<<a.n_rows, QT, 0, st>>>(a); break;
+    case ACT_PLAIN: quantize_kernel<ACT_PLAIN><<<grid, QT, 0, st>>>(a); break;
     case ACT_RMSNORM: {
         const size_t smem = ((size_t)a.dim + a.dim / 16 + 16) * 4;
         static PerDeviceOnce once;
@@ -159,7 +164,7 @@ void launch_quantize(int source, const QuantArgs &args, cudaStream_t st) {
         quantize_kernel<ACT_RMSNORM><<<a.n_rows, QT, smem, st>>>(a);
         break;
     }
-    default: quantize_kernel<ACT_SWIGLU><<<a.n_rows, QT, 0, st>>>(a); break;
+    default: quantize_kernel<ACT_SWIGLU><<<grid, QT, 0, st>>>(a); break;
     }
 }
 
