@@ -193,7 +193,7 @@ gemm_tc5_q8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 // back: 14336 x 4096 with 512 tokens 213 us in prefill order (now 132), 4096 x 14336 with 64 tokens 70 us in decode order on mma.sync
 // tiles (now 55).  What bounds this form is instruction issue: five warps share a scheduler, and a super-block's expansion, epilogue and
 // product issue are some 250 instructions each.
-constexpr int KQ_EPI_WARPS = 8, KQ_EXP_WARPS = 8, KQ_TMA_WARP = 16, KQ_MMA_WARP = 17, KQ_THREADS = 18 * 32;
+constexpr int KQ_EPI_WARPS = 8, KQ_EXP_WARPS = 8, KQ_TMA_WARP = 16, KQ_MMA_WARP = 17, KQ_THREADS = 19 * 32;
 constexpr uint32_t KQ_RAW_BYTES = TC_M * 144, KQ_A_COLS = 128;
 // TWO: the halves of a super-block have accumulators of their own (matrices with many wide rows).
 template <bool GEMM, int N>
@@ -268,6 +268,11 @@ struct Ring {
             at = 0;
             ++round;
         }
+    }
+    __device__ __forceinline__ void skip(uint32_t n) {
+        at += n;
+        round += at / S;
+        at %= S;
     }
     __device__ __forceinline__ uint32_t full_parity() const { return round & 1u; }
     __device__ __forceinline__ uint32_t empty_parity() const { return (round & 1u) ^ 1u; }  // of the round before
@@ -367,7 +372,12 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_tc5_q4k_kernel(const __gri
                 }
             }
         }
-    } else if (warp == KQ_MMA_WARP) {
+    } else if (warp >= KQ_MMA_WARP) {
+        // Two warps issue, on schedulers of their own: the first all mins, then each every other super-block.  A warp goes through the phases
+        // of its barriers one by one: it waits for a slot's, a buffer's or a stage's n-th use only when the one before is known to be over
+        // (by its own waits, by the epilogue's order, or by the meeting points before and after the mins).
+        const uint32_t which = warp - KQ_MMA_WARP;
+        auto meet = [] { asm volatile("bar.sync 1, 64;" ::: "memory"); };
         constexpr uint32_t idesc = umma_idesc_f16(N), BOX = N * 128 / 16;
         Ring<P::B_STAGES> bs;
         Ring<2> ab, ac;
@@ -384,23 +394,36 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_tc5_q4k_kernel(const __gri
             ab.next();
             bs.next();
         };
-        for (uint32_t tile = blockIdx.x; tile < a.n_tiles && ok; tile += gridDim.x) {
-            for (uint32_t j = 0; j < n_min && ok; ++j) {  // sixteen super-blocks of mins
-                if (!(ok = wait_operands())) break;
-                const uint64_t db = umma_desc_sw128(sbase + P::B + bs.at * P::B_STAGE);
-                const uint32_t ta = tmem + P::A_COL + ab.at * KQ_A_COLS;
-                for (uint32_t i = 0; i < 16 && 16 * j + i < nb; ++i) {
-                    if (!(ok = wait_slot())) break;
-                    tc_fence_after();
-                    const uint32_t td = tmem + ac.at * P::SLOT_COLS;
-                    const uint64_t d = db + (i >> 2) * BOX + (i & 3u) * 2;
-                    umma_bf16_ta_warp(td, ta + 8 * i, d, idesc, 0u);
-                    umma_commit_warp(sbase + P::ACC_FULL + 8 * ac.at);
-                    ac.next();
+        for (uint32_t tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x) {  // (after a failed wait too: both warps come to every meeting)
+            if (GEMM) {
+                if (which == 0) {
+                    for (uint32_t j = 0; j < n_min && ok; ++j) {  // sixteen super-blocks of mins
+                        if (!(ok = wait_operands())) break;
+                        const uint64_t db = umma_desc_sw128(sbase + P::B + bs.at * P::B_STAGE);
+                        const uint32_t ta = tmem + P::A_COL + ab.at * KQ_A_COLS;
+                        for (uint32_t i = 0; i < 16 && 16 * j + i < nb; ++i) {
+                            if (!(ok = wait_slot())) break;
+                            tc_fence_after();
+                            umma_bf16_ta_warp(tmem + ac.at * P::SLOT_COLS, ta + 8 * i, db + (i >> 2) * BOX + (i & 3u) * 2, idesc, 0u);
+                            umma_commit_warp(sbase + P::ACC_FULL + 8 * ac.at);
+                            ac.next();
+                        }
+                        if (ok) stage_done();
+                    }
+                } else {
+                    ab.skip(n_min);
+                    bs.skip(n_min);
+                    ac.skip(nb);
                 }
-                if (ok) stage_done();
+                meet();
             }
             for (uint32_t s = 0; s < nb && ok; ++s) {
+                if (TWO ? which == 1 : (s & 1u) != which) {  // (halves apart take both slots: one warp issues them all)
+                    ab.next();
+                    bs.next();
+                    ac.skip(TWO ? 2 : 1);
+                    continue;
+                }
                 const uint32_t ta = tmem + P::A_COL + ab.at * KQ_A_COLS;
                 const uint64_t db = umma_desc_sw128(sbase + P::B + bs.at * P::B_STAGE);
                 if (!(ok = wait_slot() && wait_operands())) break;
@@ -420,6 +443,7 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_tc5_q4k_kernel(const __gri
                 stage_done();
                 ac.next();
             }
+            meet();
         }
     } else if (warp >= KQ_EPI_WARPS) {
         // ---- expanders: thread = half a super-block of one row
