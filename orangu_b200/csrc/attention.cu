@@ -1198,6 +1198,7 @@ __global__ void __launch_bounds__(G * 16) attn_output_kernel(AttnExactArgs a) {
         const AoTile<G> &tl = tiles[t & 1];
         const uint32_t cnt = min(AO_P, n_pos - t * AO_P);
         uint32_t p = 0;
+#pragma unroll 4
         for (; p + 8 <= cnt; p += 8) {  // the products of eight positions first, so that the chain is additions alone
             const float4 wa = *reinterpret_cast<const float4 *>(&tl.w[g][p]), wb = *reinterpret_cast<const float4 *>(&tl.w[g][p + 4]);
             const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};

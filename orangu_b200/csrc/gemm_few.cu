@@ -21,15 +21,16 @@ namespace {
 
 constexpr int FW_WARPS = 8, FW_ROWS = 16;
 
+// c = a b (the accumulator goes in as zeros, which costs no registers)
 __device__ __forceinline__ void mma_u8s8_k32(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                 : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
 }
 __device__ __forceinline__ void mma_s8s8_k16(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
-                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
-                 : "r"(a0), "r"(a1), "r"(b0));
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+                 : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+                 : "r"(a0), "r"(a1), "r"(b0), "r"(0));
 }
 __device__ __forceinline__ int dp2a_lo_su(uint32_t a, uint32_t b, int c) {  // c + a.lo16 * b.byte0 + a.hi16 * b.byte1 (a signed, b unsigned)
     int d;
@@ -83,6 +84,9 @@ __global__ void __launch_bounds__(FW_WARPS * 32, 2) gemm_few_kernel(const __grid
     // ---- the copies: where this warp's ring is being filled
     uint32_t c_tile = blockIdx.x, c_b = warp, c_stage = 0, c_tok0 = 0;
     const uint8_t *src[P::COPIES];
+    const int8_t *x_src[4 * NT];  // two tokens a round
+    const int16_t *s_src = nullptr;
+    const float *d_src = nullptr;
     auto aim = [&] {
         if (c_tile >= n_tiles) return;
         uint32_t row0;
@@ -92,21 +96,24 @@ __global__ void __launch_bounds__(FW_WARPS * 32, 2) gemm_few_kernel(const __grid
             const uint32_t c = min(32 * i + lane, FW_ROWS * P::PIECES - 1), r = c / P::PIECES;
             src[i] = w.data + (uint64_t)row_of(w, row0 + r) * w.row_stride + (c - r * P::PIECES) * 16;
         }
+#pragma unroll
+        for (uint32_t i = 0; i < 4 * NT; ++i) x_src[i] = a.act.q + (uint64_t)min(c_tok0 + 2 * i + (lane >> 4), last) * a.act.dim_cap + (lane & 15) * 16;
+        s_src = a.act.sums + (uint64_t)min(c_tok0 + lane / 2, last) * (a.act.dim_cap / 16) + (lane & 1) * 8;  // (tokens 0-15: two pieces each)
+        d_src = a.act.d + (uint64_t)min(c_tok0 + lane, last) * (a.act.dim_cap / 256);
     };
     auto cp16 = [](uint32_t dst, const void *from) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(from) : "memory"); };
+    // (Places of tokens past the end hold anything: what comes of them is not stored.  Copies of the last token instead made 2 tokens slower
+    // than 8, every CTA asking for the same lines seven times over.)
     auto copy = [&] {  // the next super-block of this warp, or an empty group
         if (c_tile < n_tiles && c_b < nb) {
             const uint32_t st = (uint32_t)__cvta_generic_to_shared(ring + c_stage * P::STAGE), dst = st + lane * 16;
 #pragma unroll
-            for (uint32_t i = 0; i < 4 * NT; ++i) {  // two tokens a round
-                const uint32_t t = 2 * i + (lane >> 4), j = lane & 15;
-                cp16(st + P::X + t * 256 + ((j ^ (t & 7u)) * 16), a.act.q + (uint64_t)min(c_tok0 + t, last) * a.act.dim_cap + c_b * 256 + j * 16);
+            for (uint32_t i = 0; i < 4 * NT; ++i) {
+                const uint32_t t = 2 * i + (lane >> 4), k = lane & 15;
+                if (c_tok0 + t <= last) cp16(st + P::X + t * 256 + ((k ^ (t & 7u)) * 16), x_src[i] + c_b * 256);
             }
-            if (TYPE == TYPE_Q4_K && lane < 2 * TOK) {
-                for (uint32_t i = lane; i < 2 * TOK; i += 32) cp16(st + P::S16 + i * 16, a.act.sums + (uint64_t)min(c_tok0 + i / 2, last) * (a.act.dim_cap / 16) + c_b * 16 + (i & 1) * 8);
-            }
-            if (lane < TOK)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(st + P::AD + lane * 4), "l"(a.act.d + (uint64_t)min(c_tok0 + lane, last) * (a.act.dim_cap / 256) + c_b) : "memory");
+            if (TYPE == TYPE_Q4_K && lane < 2 * TOK && c_tok0 + lane / 2 <= last) cp16(st + P::S16 + lane * 16, s_src + c_b * 16);
+            if (lane < TOK && c_tok0 + lane <= last) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(st + P::AD + lane * 4), "l"(d_src + c_b) : "memory");
 #pragma unroll
             for (uint32_t i = 0; i < P::COPIES; ++i)
                 if (32 * i + lane < FW_ROWS * P::PIECES) cp16(dst + i * 512, src[i] + (uint64_t)c_b * P::BLK);
@@ -172,10 +179,10 @@ __global__ void __launch_bounds__(FW_WARPS * 32, 2) gemm_few_kernel(const __grid
                 const uint32_t M = 0x0f0f0f0fu;
                 const int g = s >> 1, sh = s & 1 ? 4 : 0;
                 const uint32_t a0 = (q[0][g].x >> sh) & M, a1 = (q[1][g].x >> sh) & M, a2 = (q[0][g].y >> sh) & M, a3 = (q[1][g].y >> sh) & M;
-                const int s0 = (int)((scw[0][s >> 2] >> (8 * (s & 3))) & 0xffu), s1 = (int)((scw[1][s >> 2] >> (8 * (s & 3))) & 0xffu);
+                const int s0 = (int)__byte_perm(scw[0][s >> 2], 0, 0x4440 + (s & 3)), s1 = (int)__byte_perm(scw[1][s >> 2], 0, 0x4440 + (s & 3));
 #pragma unroll
                 for (int n = 0; n < NT; ++n) {
-                    int c[4] = {0, 0, 0, 0};
+                    int c[4];
                     const uint2 x = *reinterpret_cast<const uint2 *>(x_at(n, 32 * s + 8 * tig));
                     mma_u8s8_k32(c, a0, a1, a2, a3, x.x, x.y);
                     isum[n][0] += s0 * c[0];
@@ -249,7 +256,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32, 2) gemm_few_kernel(const __grid
                         const int s0 = (int)(int8_t)((w0 >> (8 * (sidx & 3))) & 0xff), s1 = (int)(int8_t)((w1 >> (8 * (sidx & 3))) & 0xff);
 #pragma unroll
                         for (int n = 0; n < NT; ++n) {
-                            int c[4] = {0, 0, 0, 0};
+                            int c[4];
                             mma_s8s8_k16(c, v[0][run], v[1][run], word(x_at(n, 128 * h + 32 * run + 16 * is + 4 * tig)));
                             isum[n][0] += s0 * c[0];
                             isum[n][1] += s0 * c[1];

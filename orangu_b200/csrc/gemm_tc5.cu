@@ -655,7 +655,7 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_tc5_q4k_kernel(const __gri
 
 bool gemm_tc5_supported(const GemvArgs &a) {
     static const bool enabled = [] { const char *e = getenv("OB_TC5"); return !(e && e[0] == '0' && e[1] == 0); }();
-    if (!enabled || a.n_seg < 1 || a.n_tokens < 16 || a.isum_out || !encode_fn()) return false;
+    if (!enabled || a.n_seg < 1 || a.n_tokens < (a.seg[0].w.type == TYPE_Q4_K ? ACT_H_ROWS : 16u) || a.isum_out || !encode_fn()) return false;
     const uint32_t type = a.seg[0].w.type, in_dim = a.seg[0].w.in_dim;
     if (type == TYPE_Q8_0) {
         if (in_dim % 128 || a.act.dim_cap % 128) return false;

@@ -454,11 +454,16 @@ void launch_gemv(const GemvArgs &a, int sm_count, cudaStream_t st) {
     static const bool use_mma = [] { const char *e = getenv("OB_MMA"); return !(e && e[0] == '0' && e[1] == 0); }();
     const bool tc5 = gemm_tc5_supported(a);
     if (gemm_few_supported(a)) {
-        // A few tokens (gemm_few.cu).  Against tcgen05 tiles by what both take; Q6_K has none, and its 64-row tiles (gemm_mma.cu) overtake
-        // at 32768 x 4096 with 17 tokens (72 us against 108), at 4096 x 14336 with 33 (86 against 88).
+        // A few tokens (gemm_few.cu), against tcgen05 tiles by what both take.  Q6_K has none, and its 64-row tiles (gemm_mma.cu) overtake at
+        // 14336 x 4096 with 9 tokens (33 us against 35), at 32768 x 4096 with 17 (72 against 108), at 4096 x 14336 with 33 (86 against 88).
+        // With 2 or 3 tokens and more than two rounds of tiles the dp4a kernel below is ahead (14336 x 4096, 2 tokens: 23 us against 25).
         uint32_t rows = 0;
         for (int s = 0; s < a.n_seg; ++s) rows += a.seg[s].w.out_dim;
-        const bool few = tc5 ? gemm_few_us(a) < gemm_tc5_q4k_us(a, sm_count) : a.n_tokens <= 16 || (a.n_tokens <= 32 && rows <= 8192);
+        const bool rounds = rows > 2 * 16 * 2 * (uint32_t)sm_count;
+        bool few;
+        if (rounds && a.n_tokens <= 3) few = false;
+        else if (tc5) few = gemm_few_us(a) < gemm_tc5_q4k_us(a, sm_count);
+        else few = a.n_tokens <= (rounds ? 8u : 16u) || (a.n_tokens <= 32 && rows <= 8192);
         if (few && launch_gemm_few(a, sm_count, st)) return;
     }
     if (tc5 && launch_gemm_tc5(a, sm_count, st)) return;  // many tokens: tcgen05 tiles (gemm_tc5.cu)

@@ -33,7 +33,7 @@ struct ActBuf {
     float *dt = nullptr;     // [dim/256][dt_pitch] d with the rows side by side
     uint32_t dt_pitch = 0;   // a multiple of 4
 };
-constexpr uint32_t ACT_H_ROWS = 16;
+constexpr uint32_t ACT_H_ROWS = 9;
 enum ActSource { ACT_PLAIN = 0, ACT_RMSNORM = 1, ACT_SWIGLU = 2 };
 struct QuantArgs {
     const float *x;       // [n_rows][dim]   (PLAIN, RMSNORM) or gate (SWIGLU)
@@ -83,7 +83,7 @@ OB_QUANT bool launch_gemm_few_rows(const GemvArgs &a, int segment, int sm_count,
 OB_QUANT bool gemm_mma_supported(const GemvArgs &a);
 OB_QUANT void launch_gemm_mma(const GemvArgs &a, int sm_count, cudaStream_t st);
 
-// ---- gemm_tc5.cu: many-token products on tcgen05 tensor cores with TMEM accumulators, TMA-fed (16 tokens or more)
+// ---- gemm_tc5.cu: many-token products on tcgen05 tensor cores with TMEM accumulators, TMA-fed (Q8_0 16 tokens or more, Q4_K ACT_H_ROWS)
 OB_QUANT bool gemm_tc5_supported(const GemvArgs &a);
 OB_QUANT bool launch_gemm_tc5(const GemvArgs &a, int sm_count, cudaStream_t st);  // false: a tensor map could not be made (nothing was launched)
 OB_QUANT double gemm_tc5_q4k_us(const GemvArgs &a, int sm_count);  // about how long it takes
