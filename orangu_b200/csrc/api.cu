@@ -181,7 +181,7 @@ int make_weight(ob_ctx *ctx, const uint8_t *raw, uint64_t row_bytes, uint32_t ty
         cudaMemsetAsync(wide, 0, wide_bytes, ctx->stream);
         launch_q4k_wide(d, wide, ctx->stream);
         ctx->launches++;
-        d.wide = wide;
+        w->wide.flags = wide;
         std::vector<uint8_t> flags(n_rows);
         std::vector<uint32_t> rows;
         e = cudaMemcpyAsync(flags.data(), wide, n_rows, cudaMemcpyDeviceToHost, ctx->stream);
@@ -189,9 +189,9 @@ int make_weight(ob_ctx *ctx, const uint8_t *raw, uint64_t row_bytes, uint32_t ty
         if (e == cudaSuccess) {
             for (uint32_t r = 0; r < n_rows; ++r)
                 if (flags[r]) rows.push_back(r);
-            d.n_wide = (uint32_t)rows.size();
-            d.wide_rows = reinterpret_cast<const uint32_t *>(wide + wide_bytes);
-            if (d.n_wide) e = cudaMemcpyAsync(wide + wide_bytes, rows.data(), rows.size() * 4, cudaMemcpyHostToDevice, ctx->stream);
+            w->wide.n = (uint32_t)rows.size();
+            w->wide.rows = reinterpret_cast<const uint32_t *>(wide + wide_bytes);
+            if (w->wide.n) e = cudaMemcpyAsync(wide + wide_bytes, rows.data(), rows.size() * 4, cudaMemcpyHostToDevice, ctx->stream);
         }
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);  // the vectors go
     }
@@ -316,6 +316,7 @@ int matmul_device(ob_ctx *ctx, const float *x_dev, uint32_t n_tokens, const ob_w
     a.x_f32 = fused_q8 ? x_dev : nullptr;
     a.n_seg = 1;
     a.seg[0].w = w->w;
+    a.seg[0].wide = &w->wide;
     if (isum_out) {  // row window for the partial-sum capture
         a.seg[0].w.data += (uint64_t)first_row * w->w.row_stride;
         a.seg[0].w.out_dim = n_rows;

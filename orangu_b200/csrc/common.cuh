@@ -116,10 +116,13 @@ struct DevWeight {
     uint32_t nb;          // blocks per row
     uint32_t d_off;       // byte offset of the f16 d plane inside a row (Q6_K, Q8_0)
     uint64_t row_stride;  // bytes
-    // Q4_K: wide rows, with a block whose sub-block scales times codes add up to more than Q4K_SUM24: a byte per row, and the rows' numbers
-    const uint8_t *wide = nullptr;
-    const uint32_t *wide_rows = nullptr;
-    uint32_t n_wide = 0;
+};
+// Q4_K: wide rows, with a block whose sub-block scales times codes add up to more than Q4K_SUM24.  Kept beside the weight and not in
+// DevWeight: kernels of single tokens take several of those as arguments.
+struct WideRows {
+    const uint8_t *flags = nullptr;   // device: a byte per row
+    const uint32_t *rows = nullptr;   // device: the rows' numbers
+    uint32_t n = 0;
 };
 // 256 products of other blocks with 8-bit activations add up to whole numbers below 2^24, whatever the activations
 constexpr uint32_t Q4K_SUM24 = ((1u << 24) - 1) / 127;

@@ -357,10 +357,10 @@ bool launch_gemm_few_rows(const GemvArgs &a, int segment, int sm_count, cudaStre
     GemvArgs one = a;
     one.n_seg = 1;
     one.seg[0] = a.seg[segment];
-    const DevWeight &w = one.seg[0].w;
-    const bool two = few_smem(TYPE_Q4_K, w.nb, a.gemm_order, 2) <= 226 * 1024;
-    if (a.gemm_order) return two ? launch_few<TYPE_Q4_K, true, 2>(one, sm_count, st, w.wide_rows, w.n_wide) : launch_few<TYPE_Q4_K, true, 1>(one, sm_count, st, w.wide_rows, w.n_wide);
-    return two ? launch_few<TYPE_Q4_K, false, 2>(one, sm_count, st, w.wide_rows, w.n_wide) : launch_few<TYPE_Q4_K, false, 1>(one, sm_count, st, w.wide_rows, w.n_wide);
+    const WideRows &wide = *one.seg[0].wide;
+    const bool two = few_smem(TYPE_Q4_K, one.seg[0].w.nb, a.gemm_order, 2) <= 226 * 1024;
+    if (a.gemm_order) return two ? launch_few<TYPE_Q4_K, true, 2>(one, sm_count, st, wide.rows, wide.n) : launch_few<TYPE_Q4_K, true, 1>(one, sm_count, st, wide.rows, wide.n);
+    return two ? launch_few<TYPE_Q4_K, false, 2>(one, sm_count, st, wide.rows, wide.n) : launch_few<TYPE_Q4_K, false, 1>(one, sm_count, st, wide.rows, wide.n);
 }
 
 }  // namespace ob

@@ -216,6 +216,7 @@ struct KqMaps {
 };
 struct KqArgs {
     GemvSegment seg[3];  // matrices of one width that read the same activations
+    const uint8_t *wide[3];
     uint32_t tiles[3];   // running sums of their row tiles
     uint32_t n_tokens, nb, tok_tiles, n_tiles, n_xd;
     uint64_t ones;       // F2_ONES
@@ -527,7 +528,8 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_tc5_q4k_kernel(const __gri
         bool ok = true;
         for (uint32_t tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x, ++it) {
             uint32_t row0, tok0;
-            const GemvSegment &seg = a.seg[locate(tile, row0, tok0)];
+            const uint32_t si = locate(tile, row0, tok0);
+            const GemvSegment &seg = a.seg[si];
             const uint32_t row = row0 + rl;
             const uint8_t *wrow = seg.w.data + (uint64_t)min(row, seg.w.out_dim - 1) * seg.w.row_stride;
             const uint32_t xs = it % a.n_xd, xr = it / a.n_xd;
@@ -624,7 +626,7 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_tc5_q4k_kernel(const __gri
             if (!ok) break;
             __syncwarp();
             if (lane == 0) mbar_arrive(sbase + P::XD_EMPTY + 8 * xs);
-            if (row < seg.w.out_dim && (TWO || !__ldg(seg.w.wide + row))) {  // (wide rows are left to the kernel that follows)
+            if (row < seg.w.out_dim && (TWO || !__ldg(a.wide[si] + row))) {  // (wide rows are left to the kernel that follows)
                 const uint32_t t0 = tok0 + half * TPT, n = a.n_tokens > t0 ? min((uint32_t)TPT, a.n_tokens - t0) : 0u;
                 float *y = seg.y + (uint64_t)t0 * seg.y_stride + row;
                 const float *res = seg.epilogue == EPI_ADD_RESIDUAL ? seg.residual + (uint64_t)t0 * seg.y_stride + row : nullptr;
@@ -661,6 +663,8 @@ bool gemm_tc5_supported(const GemvArgs &a) {
         if (in_dim % 128 || a.act.dim_cap % 128) return false;
     } else if (type == TYPE_Q4_K) {
         if (in_dim % 256 || in_dim / 256 > 256 || !a.act.h || a.act.dim_cap % 256) return false;
+        for (int s = 0; s < a.n_seg; ++s)
+            if (!a.seg[s].wide || !a.seg[s].wide->flags) return false;
     } else {
         return false;  // Q6_K stays on the mma.sync tiles (gemm_mma.cu)
     }
@@ -687,6 +691,7 @@ static bool launch_q4k_instance(const GemvArgs &a, int sm_count, cudaStream_t st
     for (int s = 0; s < 3; ++s) {
         const int used = std::min(s, a.n_seg - 1);
         k.seg[s] = a.seg[used];
+        k.wide[s] = a.seg[used].wide->flags;
         const DevWeight &w = k.seg[s].w;
         if (!make_map_2d(&m.raw[s], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w.data, (uint64_t)nb * 144, w.out_dim, w.row_stride, 144, TC_M, CU_TENSOR_MAP_SWIZZLE_NONE)) return false;
         if (s < a.n_seg) row_tiles += (w.out_dim + TC_M - 1) / TC_M;
@@ -701,7 +706,7 @@ static bool launch_q4k_instance(const GemvArgs &a, int sm_count, cudaStream_t st
     // before the first of them started.
     bool beside = false;
     for (int s = 0; s < a.n_seg && !TWO; ++s) {
-        if (!a.seg[s].w.n_wide) continue;
+        if (!a.seg[s].wide->n) continue;
         if (!launch_gemm_few_rows(a, s, sm_count, st)) return false;
         beside = true;
     }
@@ -724,8 +729,8 @@ static KqChoice choose_q4k(const GemvArgs &a, int sm_count) {
     bool wide = false;
     for (int s = 0; s < a.n_seg; ++s) {
         const DevWeight &w = a.seg[s].w;
-        wide = wide || w.n_wide;
-        best.two = best.two || w.n_wide > (gemm_few_rows_supported(a) ? w.out_dim / 128 : 0u);
+        wide = wide || a.seg[s].wide->n;
+        best.two = best.two || a.seg[s].wide->n > (gemm_few_rows_supported(a) ? w.out_dim / 128 : 0u);
     }
     uint32_t rows = 0;
     for (int s = 0; s < a.n_seg; ++s) rows += (a.seg[s].w.out_dim + TC_M - 1) / TC_M;

@@ -16,7 +16,7 @@ namespace ob {
 // ---- formats.cu
 // src_type: the GGUF type of `src`; w.type is what the device holds (TYPE_Q8_0 for the per-32 symmetric source types).
 OB_QUANT void launch_repack(const uint8_t *src, uint64_t src_row_bytes, uint32_t src_type, uint32_t row0, uint32_t blk0, const DevWeight &w, cudaStream_t st);
-OB_QUANT void launch_q4k_wide(const DevWeight &w, uint8_t *wide, cudaStream_t st);  // fills DevWeight::wide, which was zero
+OB_QUANT void launch_q4k_wide(const DevWeight &w, uint8_t *wide, cudaStream_t st);  // fills WideRows::flags, which were zero
 OB_QUANT void launch_dequant_rows(const DevWeight &w, uint32_t first_row, uint32_t n_rows, float *out, cudaStream_t st);
 OB_QUANT void launch_embed(const DevWeight &w, const uint32_t *tokens, uint32_t n_tokens, float *out, cudaStream_t st);
 
@@ -50,6 +50,7 @@ OB_QUANT void launch_quantize(int source, const QuantArgs &a, cudaStream_t st);
 enum GemvEpilogue { EPI_STORE = 0, EPI_ADD_RESIDUAL = 1 };
 struct GemvSegment {
     DevWeight w;
+    const WideRows *wide;  // host, Q4_K: null keeps it from the tcgen05 tiles
     float *y;              // [n_tokens][y_stride]
     const float *residual; // EPI_ADD_RESIDUAL: y = residual + product (may alias y)
     uint32_t y_stride;

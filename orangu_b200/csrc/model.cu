@@ -111,6 +111,7 @@ void run_products(ob_model *m, const ActPair &act, std::initializer_list<Product
             if (done[j] || v[j].w->w.type != v[i].w->w.type) continue;
             GemvSegment &s = a.seg[a.n_seg++];
             s.w = v[j].w->w;
+            s.wide = &v[j].w->wide;
             s.y = v[j].y;
             s.y_stride = v[j].y_stride;
             s.residual = v[j].residual;

@@ -34,6 +34,7 @@ struct ob_weight {
     DevWeight w;
     void *mem;
     uint64_t bytes;
+    WideRows wide;
 };
 
 namespace obrt {
