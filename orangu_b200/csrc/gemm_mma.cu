@@ -16,8 +16,8 @@
 // A CTA is four warps = 64 rows sharing a 64-token activation tile; the weight blocks (64 x 144 B), the activations
 // (64 x 256 B, rows padded to 272 B so the fragment loads are conflict-free), their scales and sums go through a
 // two-stage cp.async ring, one super-block per stage.  This is the legacy tensor path (mma.sync): M = 16 rows per warp
-// and K = 32 per instruction match the quant format's sub-block; the tcgen05 form (128-row tiles, TMEM accumulators)
-// would need the codes unpacked to shared memory first and is not built.
+// and K = 32 per instruction match the quant format's sub-block.  Q4_K has tcgen05 tiles (gemm_tc5.cu) and comes here only with rows
+// too long for those.
 #include <cuda_pipeline.h>
 
 #include "common.cuh"

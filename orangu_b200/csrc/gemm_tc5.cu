@@ -183,7 +183,7 @@ gemm_tc5_q8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 //                  (engine/vecdot.rs:2119-2143, 2213-2255): two sweeps over K, the first over the block headers only.
 //
 // A CTA is persistent over tiles of 128 rows x N tokens.  Its warps: 0-7 epilogue (thread = one row x N / 2 tokens, two at a time in
-// packed fp32), 8-15 expanders (thread = half a super-block of one row), 16 loads (TMA), 17 issues products.  An expander turns its half
+// packed fp32), 8-15 expanders (thread = half a super-block of one row), 16 loads (TMA), 17 and 18 issue products.  An expander turns its half
 // into 64 words of two f16 -- codes enter a mantissa by a mask, one packed multiply-add takes the offset off and the scale on -- and writes
 // them to tensor memory, where the products read their A operand: expanded weights never touch shared memory, whose bandwidth the
 // activations (B, f16 from the quantizer) already take.  The order of elements within a group of four is the one the mask leaves
