@@ -329,8 +329,7 @@ int matmul_device(ob_ctx *ctx, const float *x_dev, uint32_t n_tokens, const ob_w
     a.gemm_order = !decode && n_tokens > 1;
     a.isum_out = isum_out;
     a.imin_out = imin_out;
-    launch_gemv(a, ctx->sm_count, st);
-    ctx->launches += gemv_launches(w->w.type, w->w.in_dim, n_tokens, a.gemm_order && w->w.type != TYPE_Q8_0);
+    ctx->launches += launch_gemv(a, ctx->sm_count, st);
     return OB_OK;
 }
 

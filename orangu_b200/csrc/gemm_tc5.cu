@@ -674,26 +674,26 @@ bool gemm_tc5_supported(const GemvArgs &a) {
 }
 
 template <bool GEMM, bool TWO, int N>
-static bool launch_q4k_instance(const GemvArgs &a, int sm_count, cudaStream_t st) {
+static uint32_t launch_q4k_instance(const GemvArgs &a, int sm_count, cudaStream_t st) {
     using P = KqPlan<GEMM, N>;
     static PerDeviceOnce once;
-    if (once.run([] { return cudaFuncSetAttribute(gemm_tc5_q4k_kernel<GEMM, TWO, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); }) != cudaSuccess) return false;
+    if (once.run([] { return cudaFuncSetAttribute(gemm_tc5_q4k_kernel<GEMM, TWO, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); }) != cudaSuccess) return 0;
     const uint32_t in_dim = a.seg[0].w.in_dim, nb = in_dim / 256;
     KqArgs k{};
     KqMaps m;
     k.n_xd = P::bytes(nb, 2) <= 227 * 1024 ? 2 : 1;
-    if (P::bytes(nb, k.n_xd) > 227 * 1024) return false;
+    if (P::bytes(nb, k.n_xd) > 227 * 1024) return 0;
     if (!make_map_2d(&m.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.act.h, in_dim, a.n_tokens, (uint64_t)a.act.dim_cap * 2, 64, N, CU_TENSOR_MAP_SWIZZLE_128B) ||
         !make_map_2d(&m.bs, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.act.hs, in_dim / 16, a.n_tokens, a.act.dim_cap / 16 * 2, 64, N, CU_TENSOR_MAP_SWIZZLE_128B) ||
         !make_map_2d(&m.xd, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a.act.dt, a.n_tokens, nb, (uint64_t)a.act.dt_pitch * 4, N, nb, CU_TENSOR_MAP_SWIZZLE_NONE))
-        return false;
+        return 0;
     uint32_t row_tiles = 0;
     for (int s = 0; s < 3; ++s) {
         const int used = std::min(s, a.n_seg - 1);
         k.seg[s] = a.seg[used];
         k.wide[s] = a.seg[used].wide->flags;
         const DevWeight &w = k.seg[s].w;
-        if (!make_map_2d(&m.raw[s], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w.data, (uint64_t)nb * 144, w.out_dim, w.row_stride, 144, TC_M, CU_TENSOR_MAP_SWIZZLE_NONE)) return false;
+        if (!make_map_2d(&m.raw[s], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w.data, (uint64_t)nb * 144, w.out_dim, w.row_stride, 144, TC_M, CU_TENSOR_MAP_SWIZZLE_NONE)) return 0;
         if (s < a.n_seg) row_tiles += (w.out_dim + TC_M - 1) / TC_M;
         k.tiles[s] = row_tiles;
     }
@@ -704,17 +704,17 @@ static bool launch_q4k_instance(const GemvArgs &a, int sm_count, cudaStream_t st
     k.n_tiles = row_tiles * k.tok_tiles;
     // Wide rows first, in a kernel that lets this one start beside it: neither reads what the other writes, and both read what was complete
     // before the first of them started.
-    bool beside = false;
+    uint32_t beside = 0;
     for (int s = 0; s < a.n_seg && !TWO; ++s) {
         if (!a.seg[s].wide->n) continue;
-        if (!launch_gemm_few_rows(a, s, sm_count, st)) return false;
-        beside = true;
+        if (!launch_gemm_few_rows(a, s, sm_count, st)) return 0;
+        ++beside;
     }
     const uint32_t grid = std::min(k.n_tiles, (uint32_t)std::max(1, sm_count));
     if (beside) launch_pdl(gemm_tc5_q4k_kernel<GEMM, TWO, N>, grid, KQ_THREADS, P::bytes(nb, k.n_xd), st, m, k);
     else gemm_tc5_q4k_kernel<GEMM, TWO, N><<<grid, KQ_THREADS, P::bytes(nb, k.n_xd), st>>>(m, k);
     g_tc5_launched.store(true, std::memory_order_relaxed);
-    return true;
+    return 1 + beside;
 }
 
 // How the product of Q4_K matrices is cut: tokens per tile, whether halves are kept apart, and about how long it takes.
@@ -752,7 +752,7 @@ static KqChoice choose_q4k(const GemvArgs &a, int sm_count) {
 }
 double gemm_tc5_q4k_us(const GemvArgs &a, int sm_count) { return choose_q4k(a, std::max(1, sm_count)).us; }
 
-static bool launch_q4k(const GemvArgs &a, int sm_count, cudaStream_t st) {
+static uint32_t launch_q4k(const GemvArgs &a, int sm_count, cudaStream_t st) {
     const KqChoice c = choose_q4k(a, std::max(1, sm_count));
     if (a.gemm_order && !c.two) {
         switch (c.n) {
@@ -779,22 +779,22 @@ static bool launch_q4k(const GemvArgs &a, int sm_count, cudaStream_t st) {
         case 16: return launch_q4k_instance<false, true, 16>(a, sm_count, st);
         }
     }
-    return false;  // a row too long for any tile
+    return 0;  // a row too long for any tile
 }
 
-bool launch_gemm_tc5(const GemvArgs &a, int sm_count, cudaStream_t st) {
+uint32_t launch_gemm_tc5(const GemvArgs &a, int sm_count, cudaStream_t st) {
     if (a.seg[0].w.type == TYPE_Q4_K) return launch_q4k(a, sm_count, st);
     static PerDeviceOnce once;
-    if (once.run([] { return cudaFuncSetAttribute(gemm_tc5_q8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Q8Smem::ALLOC); }) != cudaSuccess) return false;
+    if (once.run([] { return cudaFuncSetAttribute(gemm_tc5_q8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Q8Smem::ALLOC); }) != cudaSuccess) return 0;
     const uint32_t in_dim = a.seg[0].w.in_dim;
     CUtensorMap tm_x, tm_xd;
-    if (!make_map_2d(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.act.q, in_dim, a.n_tokens, a.act.dim_cap, 128, TC_N, CU_TENSOR_MAP_SWIZZLE_128B)) return false;
+    if (!make_map_2d(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.act.q, in_dim, a.n_tokens, a.act.dim_cap, 128, TC_N, CU_TENSOR_MAP_SWIZZLE_128B)) return 0;
     if (!make_map_2d(&tm_xd, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a.act.d, in_dim / 32, a.n_tokens, (uint64_t)(a.act.dim_cap / 32) * 4, 4, TC_N, CU_TENSOR_MAP_SWIZZLE_NONE))
-        return false;
+        return 0;
     for (int s = 0; s < a.n_seg; ++s) {
         const GemvSegment &g = a.seg[s];
         CUtensorMap tm_w;
-        if (!make_map_2d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, g.w.data, in_dim, g.w.out_dim, g.w.row_stride, 128, TC_M, CU_TENSOR_MAP_SWIZZLE_128B)) return false;
+        if (!make_map_2d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, g.w.data, in_dim, g.w.out_dim, g.w.row_stride, 128, TC_M, CU_TENSOR_MAP_SWIZZLE_128B)) return 0;
         TcQ8Args k{};
         k.seg = g;
         k.n_tokens = a.n_tokens;
@@ -803,7 +803,7 @@ bool launch_gemm_tc5(const GemvArgs &a, int sm_count, cudaStream_t st) {
         gemm_tc5_q8_kernel<<<grid, TC_THREADS, Q8Smem::ALLOC, st>>>(tm_w, tm_x, tm_xd, k);
         g_tc5_launched.store(true, std::memory_order_relaxed);
     }
-    return true;
+    return (uint32_t)a.n_seg;
 }
 
 int gemm_tc5_take_status() { return tc5_take_status(); }

@@ -401,9 +401,9 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_kernel(GemvArgs a, uint3
 }
 
 template <uint32_t TYPE, int T, bool GEMM>
-void launch_tile(const GemvArgs &a, int grid, size_t smem, cudaStream_t st) {
+uint32_t launch_tile(const GemvArgs &a, int grid, size_t smem, cudaStream_t st) {
     static PerDeviceOnce once;  // one per instantiation
-    if (once.run([] { return cudaFuncSetAttribute(gemv_kernel<TYPE, T, GEMM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); }) != cudaSuccess) return;
+    if (once.run([] { return cudaFuncSetAttribute(gemv_kernel<TYPE, T, GEMM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); }) != cudaSuccess) return 0;
     if (TYPE == TYPE_Q8_0 && T == 1 && a.x_f32) {  // the fused single-token form overlaps its launch with its predecessor's tail
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)grid);
@@ -416,18 +416,19 @@ void launch_tile(const GemvArgs &a, int grid, size_t smem, cudaStream_t st) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         cudaLaunchKernelEx(&cfg, gemv_kernel<TYPE, T, GEMM>, a, 0u);
-        return;
+        return 1;
     }
     for (uint32_t tok0 = 0; tok0 < a.n_tokens; tok0 += T) gemv_kernel<TYPE, T, GEMM><<<grid, GEMV_THREADS, smem, st>>>(a, tok0);
+    return (a.n_tokens + T - 1) / T;
 }
 
 template <uint32_t TYPE, bool GEMM>
-void launch_type(const GemvArgs &a, uint32_t T, int grid, size_t smem, cudaStream_t st) {
+uint32_t launch_type(const GemvArgs &a, uint32_t T, int grid, size_t smem, cudaStream_t st) {
     switch (T) {
-    case 8: launch_tile<TYPE, 8, GEMM>(a, grid, smem, st); break;
-    case 4: launch_tile<TYPE, 4, GEMM>(a, grid, smem, st); break;
-    case 2: launch_tile<TYPE, 2, GEMM>(a, grid, smem, st); break;
-    default: launch_tile<TYPE, 1, GEMM>(a, grid, smem, st); break;
+    case 8: return launch_tile<TYPE, 8, GEMM>(a, grid, smem, st);
+    case 4: return launch_tile<TYPE, 4, GEMM>(a, grid, smem, st);
+    case 2: return launch_tile<TYPE, 2, GEMM>(a, grid, smem, st);
+    default: return launch_tile<TYPE, 1, GEMM>(a, grid, smem, st);
     }
 }
 
@@ -437,19 +438,11 @@ size_t gemv_smem_bytes(uint32_t type, uint32_t in_dim, uint32_t tile_tokens, boo
     return smem_plan(type, in_dim, tile_tokens, gemm_order).total;
 }
 
-uint32_t gemv_launches(uint32_t type, uint32_t in_dim, uint32_t n_tokens, bool gemm_order) {
-    if (type == TYPE_Q5_K) return 1;
-    if ((type == TYPE_Q4_K || type == TYPE_Q6_K) && n_tokens >= 2) return 1;  // the tensor-core kernels cover all tokens in one launch (wide rows apart)
-    uint32_t T = 8;
-    while (T > 1 && (T / 2 >= n_tokens || gemv_smem_bytes(type, in_dim, T, gemm_order) > 200 * 1024)) T /= 2;
-    return (n_tokens + T - 1) / T;
-}
-
-void launch_gemv(const GemvArgs &a, int sm_count, cudaStream_t st) {
-    if (a.n_tokens == 0 || a.n_seg == 0) return;
+uint32_t launch_gemv(const GemvArgs &a, int sm_count, cudaStream_t st) {
+    if (a.n_tokens == 0 || a.n_seg == 0) return 0;
     if (a.seg[0].w.type == TYPE_Q5_K) {  // its own kernel, both orders (q5k.cu)
         launch_q5k(a, sm_count, st);
-        return;
+        return 1;
     }
     static const bool use_mma = [] { const char *e = getenv("OB_MMA"); return !(e && e[0] == '0' && e[1] == 0); }();
     const bool tc5 = gemm_tc5_supported(a);
@@ -464,12 +457,14 @@ void launch_gemv(const GemvArgs &a, int sm_count, cudaStream_t st) {
         if (rounds && a.n_tokens <= 3) few = false;
         else if (tc5) few = gemm_few_us(a) < gemm_tc5_q4k_us(a, sm_count);
         else few = a.n_tokens <= (rounds ? 8u : 16u) || (a.n_tokens <= 32 && rows <= 8192);
-        if (few && launch_gemm_few(a, sm_count, st)) return;
+        if (few && launch_gemm_few(a, sm_count, st)) return 1;
     }
-    if (tc5 && launch_gemm_tc5(a, sm_count, st)) return;  // many tokens: tcgen05 tiles (gemm_tc5.cu)
+    if (tc5) {  // many tokens: tcgen05 tiles (gemm_tc5.cu)
+        if (const uint32_t n = launch_gemm_tc5(a, sm_count, st)) return n;
+    }
     if (use_mma && gemm_mma_supported(a)) {  // many tokens: tensor-core tiles (gemm_mma.cu)
         launch_gemm_mma(a, sm_count, st);
-        return;
+        return 1;
     }
     const uint32_t type = a.seg[0].w.type, in_dim = a.seg[0].w.in_dim;
     // Q8_0's two orders are the same arithmetic; Q4_K / Q6_K differ only when asked for the GEMM order.
@@ -482,14 +477,11 @@ void launch_gemv(const GemvArgs &a, int sm_count, cudaStream_t st) {
     while (T > 1 && (T / 2 >= a.n_tokens || gemv_smem_bytes(type, in_dim, T, gemm) > budget)) T /= 2;
     const size_t smem = gemv_smem_bytes(type, in_dim, T, gemm);
     if (type == TYPE_Q4_K) {
-        if (gemm) launch_type<TYPE_Q4_K, true>(a, T, grid, smem, st);
-        else launch_type<TYPE_Q4_K, false>(a, T, grid, smem, st);
+        return gemm ? launch_type<TYPE_Q4_K, true>(a, T, grid, smem, st) : launch_type<TYPE_Q4_K, false>(a, T, grid, smem, st);
     } else if (type == TYPE_Q6_K) {
-        if (gemm) launch_type<TYPE_Q6_K, true>(a, T, grid, smem, st);
-        else launch_type<TYPE_Q6_K, false>(a, T, grid, smem, st);
-    } else {
-        launch_type<TYPE_Q8_0, false>(a, T, grid, smem, st);
+        return gemm ? launch_type<TYPE_Q6_K, true>(a, T, grid, smem, st) : launch_type<TYPE_Q6_K, false>(a, T, grid, smem, st);
     }
+    return launch_type<TYPE_Q8_0, false>(a, T, grid, smem, st);
 }
 
 }  // namespace ob

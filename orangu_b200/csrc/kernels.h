@@ -66,9 +66,8 @@ struct GemvArgs {
     int32_t *isum_out;     // optional debug capture (single segment, token 0): [out_dim][nb]
     int32_t *imin_out;
 };
-OB_QUANT void launch_gemv(const GemvArgs &a, int sm_count, cudaStream_t st);
+OB_QUANT uint32_t launch_gemv(const GemvArgs &a, int sm_count, cudaStream_t st);  // kernels launched
 OB_QUANT size_t gemv_smem_bytes(uint32_t type, uint32_t in_dim, uint32_t tile_tokens, bool gemm_order);
-OB_QUANT uint32_t gemv_launches(uint32_t type, uint32_t in_dim, uint32_t n_tokens, bool gemm_order);  // kernels launch_gemv issues
 
 // ---- q5k.cu: Q5_K weights, one kernel for any token count and both fp32 orders
 OB_QUANT void launch_q5k(const GemvArgs &a, int sm_count, cudaStream_t st);
@@ -86,7 +85,7 @@ OB_QUANT void launch_gemm_mma(const GemvArgs &a, int sm_count, cudaStream_t st);
 
 // ---- gemm_tc5.cu: many-token products on tcgen05 tensor cores with TMEM accumulators, TMA-fed (Q8_0 16 tokens or more, Q4_K ACT_H_ROWS)
 OB_QUANT bool gemm_tc5_supported(const GemvArgs &a);
-OB_QUANT bool launch_gemm_tc5(const GemvArgs &a, int sm_count, cudaStream_t st);  // false: a tensor map could not be made (nothing was launched)
+OB_QUANT uint32_t launch_gemm_tc5(const GemvArgs &a, int sm_count, cudaStream_t st);  // kernels launched; 0: a tensor map could not be made, or a row is too long
 OB_QUANT double gemm_tc5_q4k_us(const GemvArgs &a, int sm_count);  // about how long it takes
 OB_QUANT int gemm_tc5_take_status();  // 1 when a bounded wait inside one of these kernels ran out since the last call
 

@@ -118,8 +118,7 @@ void run_products(ob_model *m, const ActPair &act, std::initializer_list<Product
             s.epilogue = v[j].residual ? EPI_ADD_RESIDUAL : EPI_STORE;
             done[j] = true;
         }
-        launch_gemv(a, m->ctx->sm_count, st);
-        m->ctx->launches += gemv_launches(a.seg[0].w.type, a.seg[0].w.in_dim, n_tokens, gemm_order && a.seg[0].w.type != TYPE_Q8_0);
+        m->ctx->launches += launch_gemv(a, m->ctx->sm_count, st);
     }
 }
 

@@ -24,6 +24,18 @@ def rel_err(got, want, magnitude):
     return float(np.max(np.abs(np.asarray(got, np.float64) - np.asarray(want, np.float64)) / np.maximum(magnitude, 1e-6)))
 
 
+def kernels_run(fn):
+    """Names of the kernels that `fn` runs on the device, with their template arguments."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        fn()
+        torch.cuda.synchronize()
+    return [e.name for e in p.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+
+
 # ---- models given as a list of layers
 def error(got, want):
     """Worst position: root mean square of the difference over the root mean square of all expected values."""
