@@ -151,6 +151,7 @@ SIGNATURES = {
     "ob_last_hidden": (_i32, [_vp, _u32, _vp]),
     "ob_launch_count": (_u64, [_vp]),
     "ob_last_device_ms": (_f32, [_vp]),
+    "ob_tile_wait_selftest": (_i32, [_vp]),
     "ob_tp_unique_id": (_i32, [_vp]),
     "ob_tp_exchange_selftest": (_i32, [_vp, _u32, _u32, _u32, _vp, _vp]),
     "ob_tp_rendezvous_selftest": (_i32, [_vp, _u32, _u32, _u32, _u32, _vp]),

@@ -110,6 +110,18 @@ void ob_destroy(ob_ctx *ctx) {
     delete ctx;
 }
 
+int ob_tile_wait_selftest(ob_ctx *ctx) {
+    if (!quantized_built()) return fail(ctx, OB_ERR_UNSUPPORTED, "tile_wait_selftest: the library was built without the quantized kernels");
+    if (!ctx) return OB_ERR_INVALID;
+    std::lock_guard<std::mutex> g(ctx->mu);
+    Bind b(ctx);
+    launch_tc5_wait_selftest(ctx->stream);
+    ctx->launches++;
+    OB_CUDA(ctx, cudaGetLastError());
+    OB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return OB_OK;
+}
+
 int ob_synchronize(ob_ctx *ctx) {
     if (!ctx) return OB_ERR_INVALID;
     Bind b(ctx);

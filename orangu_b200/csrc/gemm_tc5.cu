@@ -807,5 +807,23 @@ uint32_t launch_gemm_tc5(const GemvArgs &a, int sm_count, cudaStream_t st) {
 }
 
 int gemm_tc5_take_status() { return tc5_take_status(); }
+void gemm_tc5_mark_launched() { g_tc5_launched.store(true, std::memory_order_relaxed); }
+
+namespace {
+// A barrier that nothing arrives at, waited for by every lane of a warp with a short limit: the status word is then what a product whose
+// wait ran out leaves.
+__global__ void __launch_bounds__(32) wait_selftest_kernel() {
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t abort;
+    if (threadIdx.x == 0) {
+        mbar_init(smem_u32(&bar), 1);
+        abort = 0u;
+    }
+    __syncwarp();
+    mbar_wait(smem_u32(&bar), 0u, &abort, 256);
+}
+}  // namespace
+
+void launch_tc5_wait_selftest(cudaStream_t st) { wait_selftest_kernel<<<1, 32, 0, st>>>(); }
 
 }  // namespace ob

@@ -1624,7 +1624,9 @@ int ob_decode_loop(ob_model *m, ob_kv *const *kvs, const uint32_t *first_tokens,
     fetch_status(m, st);
     OB_CUDA(ctx, cudaStreamSynchronize(st));
     OB_CUDA(ctx, cudaGetLastError());
-    if (m->graph) linear_mark_launched();  // the replayed steps may hold tensor-core products
+    // the replayed steps may hold tensor-core products, which the host has launched only once, when they were captured
+    if (m->graph) linear_mark_launched();
+    else if (n_seq >= ACT_H_ROWS) gemm_tc5_mark_launched();  // (fewer rows have none)
     cudaEventElapsedTime(&ctx->last_ms, ctx->ev0, ctx->ev1);
     ctx->launches += m->graph_launches[key] * n_steps;
     for (uint32_t s = 0; s < n_seq; ++s) kvs[s]->len += n_steps;

@@ -31,8 +31,8 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 // False when the wait was abandoned: this one ran out of polls, or another role's did (*abort is then set).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t *abort) {
-    for (uint32_t i = 0; i < TC_POLL_LIMIT; ++i) {
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t *abort, uint32_t limit = TC_POLL_LIMIT) {
+    for (uint32_t i = 0; i < limit; ++i) {
         if (mbar_try(bar, parity)) return true;
         if ((i & 63u) == 63u && *abort) return false;
     }

@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 
 from gpu_common import backend, kernels_run  # noqa: F401
-from orangu_b200 import LlamaModel, QuantMatrix, synth
+from orangu_b200 import LlamaModel, QuantMatrix, capi, synth
 from q4k_make import q4k_blocks
 
 pytestmark = pytest.mark.gpu
@@ -24,3 +24,22 @@ def test_launches_are_counted(backend, rows, cols, n, wide):
         before = backend.launch_count()
         names = own(kernels_run(lambda: run(x, n, w)))
         assert backend.launch_count() - before == len(names), names
+
+
+@pytest.mark.parametrize("t,n_seq", [(Q4_K, 16), (Q8_0, 16)])
+def test_a_wait_that_ran_out_in_a_replayed_step_is_reported(backend, t, n_seq):
+    """The steps of a decode loop are captured at its first call and only replayed afterwards; the status that their products leave is read
+    after every call."""
+    cfg = dict(n_vocab=256, n_embd=1280, n_layer=1, n_head=10, n_head_kv=5, head_dim=128, n_ff=9472, rope_freq_base=10000.0, rms_eps=1e-5)
+    tensors = synth.model_tensors(cfg, seed=3, types={name: t for name in ("attn_q", "attn_k", "attn_v", "attn_output", "ffn_gate", "ffn_up", "ffn_down", "output")})
+    model = LlamaModel(backend, cfg, tensors, max_seq_len=64, max_batch_tokens=16, kv_pool_tokens=2048)
+    kvs = [model.new_kv_cache(48) for _ in range(n_seq)]
+    first = list(range(n_seq))
+    tile = "gemm_tc5_q4k" if t == Q4_K else "gemm_tc5_q8"
+    assert any(tile in k for k in kernels_run(lambda: model.decode_loop(kvs, first, 2)))
+    model.decode_loop(kvs, first, 2)
+    capi.check(backend._h, backend._lib.ob_tile_wait_selftest(backend._h))
+    with pytest.raises(capi.OranguError, match="gave up a bounded wait"):
+        model.decode_loop(kvs, first, 2)
+    model.decode_loop(kvs, first, 2)  # reported once
+    model.close()
