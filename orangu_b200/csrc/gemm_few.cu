@@ -308,6 +308,9 @@ size_t few_smem(uint32_t type, uint32_t nb, bool gemm, int nt) {
     return ring + (size_t)nb * FW_ROWS * 8 * nt * 4 * (gemm && type == TYPE_Q4_K ? 2 : 1);
 }
 
+// n-tiles of a CTA: 16 tokens where there are more than 8 and the terms of a tile fit beside its ring, else 8
+int few_n_tiles(const GemvArgs &a) { return a.n_tokens > 8 && few_smem(a.seg[0].w.type, a.seg[0].w.nb, a.gemm_order, 2) <= 226 * 1024 ? 2 : 1; }
+
 template <uint32_t TYPE, bool GEMM, int NT>
 bool launch_few(const GemvArgs &a, int sm_count, cudaStream_t st, const uint32_t *rows = nullptr, uint32_t n_rows = 0) {
     static PerDeviceOnce once;
@@ -336,16 +339,16 @@ bool gemm_few_supported(const GemvArgs &a) {
 }
 
 bool launch_gemm_few(const GemvArgs &a, int sm_count, cudaStream_t st) {
-    const uint32_t type = a.seg[0].w.type, nb = a.seg[0].w.nb;
-    int nt = a.n_tokens > 8 ? 2 : 1;
-    while (nt > 1 && few_smem(type, nb, a.gemm_order, nt) > 226 * 1024) nt /= 2;
+    const uint32_t type = a.seg[0].w.type;
+    const int nt = few_n_tiles(a);
     if (type == TYPE_Q4_K) return a.gemm_order ? launch_few_nt<TYPE_Q4_K, true>(a, nt, sm_count, st) : launch_few_nt<TYPE_Q4_K, false>(a, nt, sm_count, st);
     return a.gemm_order ? launch_few_nt<TYPE_Q6_K, true>(a, nt, sm_count, st) : launch_few_nt<TYPE_Q6_K, false>(a, nt, sm_count, st);
 }
 
 // Microseconds: a tile's super-block costs 1.05e-3 with 8 tokens and 1.3e-3 with 16 (4096 x 14336, 8 tokens: 18 us; 14336 x 4096, 16: 24).
+// Rows whose terms allow 8 tokens only are twice the tiles (4096 x 28672, 48 tokens, prefill order: 151 us, the tcgen05 tiles 133).
 double gemm_few_us(const GemvArgs &a) {
-    const uint32_t nt = a.n_tokens > 8 ? 2 : 1;
+    const uint32_t nt = few_n_tiles(a);
     double tiles = 0;
     for (int s = 0; s < a.n_seg; ++s) tiles += (a.seg[s].w.out_dim + FW_ROWS - 1) / FW_ROWS;
     return 5.0 + tiles * ((a.n_tokens + 8 * nt - 1) / (8 * nt)) * a.seg[0].w.nb * (nt == 1 ? 1.05e-3 : 1.3e-3);

@@ -2,7 +2,8 @@
 import numpy as np
 import pytest
 
-from gpu_common import backend, kernels_run  # noqa: F401
+import oracle as O
+from gpu_common import assert_bit_equal, backend, kernels_run  # noqa: F401
 from orangu_b200 import LlamaModel, QuantMatrix, capi, synth
 from q4k_make import q4k_blocks
 
@@ -24,6 +25,15 @@ def test_launches_are_counted(backend, rows, cols, n, wide):
         before = backend.launch_count()
         names = own(kernels_run(lambda: run(x, n, w)))
         assert backend.launch_count() - before == len(names), names
+
+
+def test_long_rows_of_many_tokens_take_the_tiles(backend):
+    """Prefill order, rows of 112 super-blocks: the few-token kernel holds the terms of 8 tokens at a time, not of 16, and is the slower."""
+    rows, cols, n = 4096, 28672, 48
+    w = QuantMatrix(q4k_blocks(rows, cols, 3, np.r_[0:0]).reshape(-1), Q4_K, cols, rows)
+    x = synth.normal(n * cols, 4)
+    assert any("gemm_tc5_q4k_kernel" in k for k in kernels_run(lambda: backend.matmul(x, n, w)))
+    assert_bit_equal(backend.matmul(x, n, w), O.matmul(x, n, w.raw, Q4_K, cols, rows), "48 tokens")
 
 
 @pytest.mark.parametrize("t,n_seq", [(Q4_K, 16), (Q8_0, 16)])
