@@ -496,9 +496,10 @@ float ob_last_device_ms(const ob_ctx *ctx);
 int ob_profile_gemv(ob_model *model, uint32_t ggml_type, uint32_t variant, uint32_t iters, float *ms_total,
                     uint64_t *bytes_per_pass, uint32_t *launches_per_pass);
 /* Diagnostic (no counterpart in the reference): every wait inside a tensor-core product is bounded, and a product that gave one up says
- * so in a word on the device, which the next call that ran such products reads and reports as OB_ERR_CUDA.  This runs a kernel whose only
- * wait is for something that never comes, with a short limit, so that the word is set; it returns OB_OK and leaves the word for the next
- * ob_matmul / ob_forward / ob_decode_loop with tensor-core products (9 rows or more) to find. */
+ * so in a word on the device, which the next call that ran such products reads and reports as OB_ERR_CUDA.  This runs a warp whose
+ * lanes wait for something that never comes, each with a short limit of its own, and then go through tensor memory together, as the
+ * warps of the products do.  The word is then set; OB_OK when all lanes went on, and the word is left for the next ob_matmul /
+ * ob_forward / ob_decode_loop with tensor-core products (9 rows or more) to find. */
 int ob_tile_wait_selftest(ob_ctx *ctx);
 
 /* --------------------------------------------------------- tensor parallel */

@@ -115,10 +115,16 @@ int ob_tile_wait_selftest(ob_ctx *ctx) {
     if (!ctx) return OB_ERR_INVALID;
     std::lock_guard<std::mutex> g(ctx->mu);
     Bind b(ctx);
-    launch_tc5_wait_selftest(ctx->stream);
+    int rc;
+    if ((rc = ensure(ctx, ctx->saux, 4))) return rc;
+    uint32_t lanes = 0;
+    OB_CUDA(ctx, cudaMemsetAsync(ctx->saux.p, 0, 4, ctx->stream));
+    launch_tc5_wait_selftest(static_cast<uint32_t *>(ctx->saux.p), ctx->stream);
     ctx->launches++;
-    OB_CUDA(ctx, cudaGetLastError());
+    OB_CUDA(ctx, cudaMemcpyAsync(&lanes, ctx->saux.p, 4, cudaMemcpyDeviceToHost, ctx->stream));
     OB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    OB_CUDA(ctx, cudaGetLastError());
+    if (lanes != 32) return fail(ctx, OB_ERR_CUDA, "tile_wait_selftest: after a wait that ran out " + std::to_string(lanes) + " of 32 lanes went on together");
     return OB_OK;
 }
 

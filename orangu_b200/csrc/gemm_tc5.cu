@@ -125,7 +125,7 @@ gemm_tc5_q8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             const uint32_t s = it % Q8_STAGES, buf = it & 1u;
             const uint2 swb = sw_next;
             if (it + 1 < n_steps) sw_next = __ldg(reinterpret_cast<const uint2 *>(wrow + 8 * (it + 1)));
-            if (!mbar_wait(sbase + Q8Smem::ACC_FULL + 8 * buf, (it / 2) & 1u, abort)) break;
+            mbar_wait_on(sbase + Q8Smem::ACC_FULL + 8 * buf, (it / 2) & 1u, abort);
             tc_fence_after();
             const float sw[4] = {f16_bits_to_f32(swb.x & 0xffffu), f16_bits_to_f32(swb.x >> 16), f16_bits_to_f32(swb.y & 0xffffu), f16_bits_to_f32(swb.y >> 16)};
             const float4 *xd = reinterpret_cast<const float4 *>(smem + Q8Smem::XD + s * Q8_XD_BYTES) + half * 32;  // [token] the four block scales
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_tc5_q4k_kernel(const __gri
             if (__all_sync(0xffffffffu, mbar_try2(x, ab.full_parity(), b, bs.full_parity()))) return true;
             return mbar_wait_warp(b, bs.full_parity(), abort) && mbar_wait_warp(x, ab.full_parity(), abort);
         };
-        auto wait_slot = [&] { return !ac.round || __all_sync(0xffffffffu, mbar_wait_ready(sbase + P::ACC_EMPTY + 8 * ac.at, ac.empty_parity(), abort)); };
+        auto wait_slot = [&] { return !ac.round || mbar_wait_ready_warp(sbase + P::ACC_EMPTY + 8 * ac.at, ac.empty_parity(), abort); };
         auto stage_done = [&] {
             umma_commit_warp(sbase + P::A_EMPTY + 8 * ab.at);
             umma_commit_warp(sbase + P::B_EMPTY + 8 * bs.at);
@@ -452,8 +452,7 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_tc5_q4k_kernel(const __gri
         const uint32_t ta = tmem + ((quad * 32) << 16) + P::A_COL;
         Ring<P::RAW_STAGES> raw;
         Ring<2> ab;
-        bool ok = true;
-        auto wait_a = [&] { return !ab.round || mbar_wait_ready(sbase + P::A_EMPTY + 8 * ab.at, ab.empty_parity(), abort); };
+        auto wait_a = [&] { if (ab.round) mbar_wait_on(sbase + P::A_EMPTY + 8 * ab.at, ab.empty_parity(), abort); };
         auto store = [&](uint32_t (&w)[64]) {
             const uint32_t to = ta + ab.at * KQ_A_COLS + 64 * h;
             tmem_st32(to, *reinterpret_cast<uint32_t(*)[32]>(w));
@@ -466,7 +465,7 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_tc5_q4k_kernel(const __gri
             if (lane == 0) mbar_arrive(sbase + P::A_FULL + 8 * ab.at);
             ab.next();
         };
-        for (uint32_t tile = blockIdx.x; tile < a.n_tiles && ok; tile += gridDim.x) {
+        for (uint32_t tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x) {
             uint32_t row0, tok0;
             const GemvSegment &seg = a.seg[locate(tile, row0, tok0)];
             const uint8_t *wrow = seg.w.data + (uint64_t)min(row0 + r, seg.w.out_dim - 1) * seg.w.row_stride;
@@ -477,14 +476,13 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_tc5_q4k_kernel(const __gri
                     const uint4 hd = __ldg(reinterpret_cast<const uint4 *>(wrow + (uint64_t)min(16 * j + 8 * h + i, nb - 1) * 144));
                     kq_mins(hd, w + 8 * i);
                 }
-                if (!(ok = wait_a())) break;
+                wait_a();
                 tc_fence_after();
                 store(w);
                 done_a();
             }
-            if (!ok) break;
             for (uint32_t s = 0; s < nb; ++s, raw.next()) {
-                if (!(ok = mbar_wait_ready(sbase + P::RAW_FULL + 8 * raw.at, raw.full_parity(), abort))) break;
+                mbar_wait_on(sbase + P::RAW_FULL + 8 * raw.at, raw.full_parity(), abort);
                 const uint8_t *blk = smem + P::RAW + raw.at * KQ_RAW_BYTES + r * 144u;
                 const uint4 hd = *reinterpret_cast<const uint4 *>(blk);
                 // the half's four 6-bit scales (engine/quant.rs:653-662) as bytes of a word, then each twice as f16
@@ -507,7 +505,7 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_tc5_q4k_kernel(const __gri
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(sbase + P::RAW_EMPTY + 8 * raw.at);
-                if (!(ok = wait_a())) break;
+                wait_a();
                 tc_fence_after();
                 store(out);
                 if (!GEMM && h == 1) {
@@ -525,7 +523,6 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_tc5_q4k_kernel(const __gri
         const uint64_t ones = a.ones;
         Ring<2> ac;
         uint32_t it = 0;
-        bool ok = true;
         for (uint32_t tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x, ++it) {
             uint32_t row0, tok0;
             const uint32_t si = locate(tile, row0, tok0);
@@ -533,7 +530,7 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_tc5_q4k_kernel(const __gri
             const uint32_t row = row0 + rl;
             const uint8_t *wrow = seg.w.data + (uint64_t)min(row, seg.w.out_dim - 1) * seg.w.row_stride;
             const uint32_t xs = it % a.n_xd, xr = it / a.n_xd;
-            if (!(ok = mbar_wait(sbase + P::XD_FULL + 8 * xs, xr & 1u, abort))) break;
+            mbar_wait_on(sbase + P::XD_FULL + 8 * xs, xr & 1u, abort);
             const float *xd = reinterpret_cast<const float *>(smem + P::XD + xs * P::xd_bytes(nb)) + half * TPT;
             uint64_t acc[TPT / 2];
 #pragma unroll
@@ -543,7 +540,7 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_tc5_q4k_kernel(const __gri
             if (GEMM) {
                 for (uint32_t s = 0; s < nb; ++s) {
                     const uint32_t dw2 = header(s + 2);
-                    if (!(ok = mbar_wait_ready(sbase + P::ACC_FULL + 8 * ac.at, ac.full_parity(), abort))) break;
+                    mbar_wait_on(sbase + P::ACC_FULL + 8 * ac.at, ac.full_parity(), abort);
                     tc_fence_after();
                     const uint64_t dmin2 = f2_both(-f16_bits_to_f32(dw0 >> 16));
                     const float4 *ad4 = reinterpret_cast<const float4 *>(xd + s * N);
@@ -570,7 +567,6 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_tc5_q4k_kernel(const __gri
                     dw0 = dw1;
                     dw1 = dw2;
                 }
-                if (!ok) break;
                 dw0 = header(0);
                 dw1 = header(1);
             }
@@ -579,10 +575,10 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_tc5_q4k_kernel(const __gri
                     const uint32_t dw2 = header(s + 2);
                     const uint64_t d2 = f2_both(f16_bits_to_f32(dw0 & 0xffffu)), dmin2 = f2_both(-f16_bits_to_f32(dw0 >> 16));
                     const uint32_t first = ac.at;
-                    if (!mbar_wait_ready(sbase + P::ACC_FULL + 8 * ac.at, ac.full_parity(), abort)) return false;
+                    mbar_wait_on(sbase + P::ACC_FULL + 8 * ac.at, ac.full_parity(), abort);
                     if (TWO) {
                         ac.next();
-                        if (!mbar_wait_ready(sbase + P::ACC_FULL + 8 * ac.at, ac.full_parity(), abort)) return false;
+                        mbar_wait_on(sbase + P::ACC_FULL + 8 * ac.at, ac.full_parity(), abort);
                     }
                     tc_fence_after();
                     const float4 *ad4 = reinterpret_cast<const float4 *>(xd + s * N);
@@ -620,13 +616,11 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) gemm_tc5_q4k_kernel(const __gri
                     dw0 = dw1;
                     dw1 = dw2;
                 }
-                return true;
             };
-            ok = sweep();
-            if (!ok) break;
+            sweep();
             __syncwarp();
             if (lane == 0) mbar_arrive(sbase + P::XD_EMPTY + 8 * xs);
-            if (row < seg.w.out_dim && (TWO || !__ldg(a.wide[si] + row))) {  // (wide rows are left to the kernel that follows)
+            if (!*abort && row < seg.w.out_dim && (TWO || !__ldg(a.wide[si] + row))) {  // (wide rows are left to the kernel that follows)
                 const uint32_t t0 = tok0 + half * TPT, n = a.n_tokens > t0 ? min((uint32_t)TPT, a.n_tokens - t0) : 0u;
                 float *y = seg.y + (uint64_t)t0 * seg.y_stride + row;
                 const float *res = seg.epilogue == EPI_ADD_RESIDUAL ? seg.residual + (uint64_t)t0 * seg.y_stride + row : nullptr;
@@ -810,20 +804,36 @@ int gemm_tc5_take_status() { return tc5_take_status(); }
 void gemm_tc5_mark_launched() { g_tc5_launched.store(true, std::memory_order_relaxed); }
 
 namespace {
-// A barrier that nothing arrives at, waited for by every lane of a warp with a short limit: the status word is then what a product whose
-// wait ran out leaves.
-__global__ void __launch_bounds__(32) wait_selftest_kernel() {
+// A barrier that nothing arrives at, waited for by every lane of a warp with a short limit of its own, then words through tensor memory, which
+// takes all lanes together: *lanes counts the lanes that got theirs back, and the status word is what a product whose wait ran out leaves.
+__global__ void __launch_bounds__(32) wait_selftest_kernel(uint32_t *lanes) {
     __shared__ __align__(8) uint64_t bar;
-    __shared__ uint32_t abort;
+    __shared__ uint32_t abort, slot;
     if (threadIdx.x == 0) {
         mbar_init(smem_u32(&bar), 1);
         abort = 0u;
     }
     __syncwarp();
-    mbar_wait(smem_u32(&bar), 0u, &abort, 256);
+    tmem_alloc(smem_u32(&slot), 32);
+    __syncwarp();
+    const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(&slot);
+    for (uint32_t i = 0; i < 2; ++i) mbar_wait_on(smem_u32(&bar), 0u, &abort, 256 + threadIdx.x);
+    uint32_t w[8], r[8];
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) w[i] = threadIdx.x * 8 + i;
+    tmem_st8(tmem, w);
+    tmem_st_wait();
+    tmem_ld8(tmem, r);
+    tmem_ld_wait();
+    bool same = true;
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) same = same && r[i] == w[i];
+    atomicAdd(lanes, same ? 1u : 0u);
+    __syncwarp();
+    tmem_dealloc(tmem, 32);
 }
 }  // namespace
 
-void launch_tc5_wait_selftest(cudaStream_t st) { wait_selftest_kernel<<<1, 32, 0, st>>>(); }
+void launch_tc5_wait_selftest(uint32_t *lanes, cudaStream_t st) { wait_selftest_kernel<<<1, 32, 0, st>>>(lanes); }
 
 }  // namespace ob

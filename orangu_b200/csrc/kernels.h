@@ -89,7 +89,7 @@ OB_QUANT uint32_t launch_gemm_tc5(const GemvArgs &a, int sm_count, cudaStream_t 
 OB_QUANT double gemm_tc5_q4k_us(const GemvArgs &a, int sm_count);  // about how long it takes
 OB_QUANT int gemm_tc5_take_status();  // 1 when a bounded wait inside one of these kernels ran out since the last call
 OB_QUANT void gemm_tc5_mark_launched();  // a replayed graph may have run one of them
-OB_QUANT void launch_tc5_wait_selftest(cudaStream_t st);
+OB_QUANT void launch_tc5_wait_selftest(uint32_t *lanes, cudaStream_t st);
 
 // ---- stream_gemv.cu: fused single-token products for decode (Q4_K / Q6_K weights)
 enum StreamPrologue { SG_PRO_PLAIN = 0, SG_PRO_RMSNORM = 1, SG_PRO_READY = 2 };

@@ -486,7 +486,7 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
             uint32_t batch, rt, tt, t0, t_end;
             lt_tile(g, tile / g.splits, &batch, &rt, &tt);
             lt_rows(g, a.T, tt, &batch, &t0, &t_end);
-            if (!mbar_wait(sbase + S::ACC_FULL + 8 * buf, (n / S::NBUF) & 1u, abort)) break;
+            if (!mbar_wait_warp(sbase + S::ACC_FULL + 8 * buf, (n / S::NBUF) & 1u, abort)) break;
             tc_fence_after();
             const uint32_t t = t0 + warp * 32 + lane;
 #pragma unroll 1

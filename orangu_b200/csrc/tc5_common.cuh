@@ -46,6 +46,17 @@ __device__ __forceinline__ bool mbar_wait_ready(uint32_t bar, uint32_t parity, v
     if (__builtin_expect(mbar_try(bar, parity), 1)) return true;
     return mbar_wait(bar, parity, abort);
 }
+// For a whole warp: all of its lanes go on or none does.  Whatever is .aligned (loads from and stores to tensor memory, their waits) may only
+// follow a wait that ended alike for every lane, also when it is given up.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t *abort) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort)); }
+// For a warp that goes through all of its loop whatever comes, so that no lane leaves before what is .aligned: once a wait was given up the
+// others are polled once, and what the warp computes is thrown away.
+__device__ __forceinline__ void mbar_wait_on(uint32_t bar, uint32_t parity, volatile uint32_t *abort, uint32_t limit = TC_POLL_LIMIT) {
+    if (!__builtin_expect(mbar_try(bar, parity), 1) && !*abort) mbar_wait(bar, parity, abort, limit);
+}
+__device__ __forceinline__ bool mbar_wait_ready_warp(uint32_t bar, uint32_t parity, volatile uint32_t *abort) {
+    return __all_sync(0xffffffffu, mbar_wait_ready(bar, parity, abort));
+}
 // Two polls in the time of little more than one.
 __device__ __forceinline__ bool mbar_try2(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1) {
     uint32_t ok;
@@ -150,7 +161,6 @@ __device__ __forceinline__ void umma_bf16_ta_warp(uint32_t d_tmem, uint32_t a_tm
 __device__ __forceinline__ void umma_commit_warp(uint32_t bar) {
     asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t *abort) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort)); }
 constexpr uint32_t UMMA_B_MN_MAJOR = 1u << 16;  // in the instruction descriptor
 // Shared-memory descriptor of an MN-major tile in the 128-byte swizzle: a row of 128 bytes holds 64 consecutive entries of one k,
 // groups of eight k 1024 bytes apart, the next 64 entries `block` bytes on.
