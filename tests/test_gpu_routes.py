@@ -36,6 +36,20 @@ def test_long_rows_of_many_tokens_take_the_tiles(backend):
     assert_bit_equal(backend.matmul(x, n, w), O.matmul(x, n, w.raw, Q4_K, cols, rows), "48 tokens")
 
 
+# 7104 and 9472 rows are one and a half times and twice what all SMs take at once; the kernels of prefill order, of decode order
+@pytest.mark.parametrize("t,rows,n,prefill,decode", [
+    (Q4_K, 7104, 2, "few", "few"), (Q4_K, 7105, 2, "gemv", "gemv"), (Q4_K, 9472, 3, "few", "few"), (Q4_K, 9473, 3, "gemv", "gemv"), (Q4_K, 9473, 4, "few", "few"),
+    (Q6_K, 9472, 2, "few", "few"), (Q6_K, 9473, 2, "few", "gemv"), (Q6_K, 9473, 3, "few", "few")])
+def test_two_and_three_tokens(backend, t, rows, n, prefill, decode):
+    cols = 768
+    w = QuantMatrix(synth.matrix(t, rows, cols, 5)["data"], t, cols, rows)
+    x = synth.normal(n * cols, 6)
+    for run, want, oracle in ((backend.matmul, prefill, O.matmul), (backend.matmul_decode, decode, O.matmul_decode)):
+        names = kernels_run(lambda: run(x, n, w))
+        assert any({"few": "gemm_few_kernel", "gemv": "gemv_kernel"}[want] in k for k in names), names
+        assert_bit_equal(run(x, n, w), oracle(x, n, w.raw, t, cols, rows), "products")
+
+
 @pytest.mark.parametrize("t,n_seq", [(Q4_K, 16), (Q8_0, 16)])
 def test_a_wait_that_ran_out_in_a_replayed_step_is_reported(backend, t, n_seq):
     """The steps of a decode loop are captured at its first call and only replayed afterwards; the status that their products leave is read
