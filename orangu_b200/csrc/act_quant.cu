@@ -147,10 +147,8 @@ __global__ void __launch_bounds__(QT) quantize_kernel(QuantArgs a) {
 
 }  // namespace
 
-void launch_quantize(int source, const QuantArgs &args, cudaStream_t st) {
-    QuantArgs a = args;
+void launch_quantize(int source, const QuantArgs &a, cudaStream_t st) {
     if (a.n_rows == 0) return;
-    if (a.n_rows < ACT_H_ROWS) a.k.h = nullptr;
     // A row of 14336 is four passes of a CTA, and the exponentials of a SwiGLU are 8 us of them one after the other: few rows are shared out
     // (9.8 us for 8 rows by a CTA each), until CTAs are two to an SM or so.
     const uint32_t passes = (a.dim + QT * 8 - 1) / (QT * 8);

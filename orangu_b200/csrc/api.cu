@@ -274,8 +274,8 @@ int ob_weight_dequantize(ob_ctx *ctx, const ob_weight *w, uint32_t first_row, ui
 
 namespace {
 
-// Quantize x_dev [n_tokens][in_dim] with the granularity `type` wants, into ctx scratch.
-int quantize_for(ob_ctx *ctx, const float *x_dev, uint32_t n_tokens, uint32_t in_dim, uint32_t type, ActBuf *act, cudaStream_t st) {
+// Quantize x_dev [n_tokens][in_dim] with the granularity `type` wants, into ctx scratch; f16: codes, sums and scales for the tcgen05 tiles too.
+int quantize_for(ob_ctx *ctx, const float *x_dev, uint32_t n_tokens, uint32_t in_dim, uint32_t type, bool f16, ActBuf *act, cudaStream_t st) {
     const uint32_t grp = type == TYPE_Q8_0 ? 32u : 256u;
     int rc;
     if ((rc = ensure(ctx, ctx->sq, (size_t)n_tokens * in_dim))) return rc;
@@ -285,7 +285,7 @@ int quantize_for(ob_ctx *ctx, const float *x_dev, uint32_t n_tokens, uint32_t in
     act->d = static_cast<float *>(ctx->sd.p);
     act->sums = static_cast<int16_t *>(ctx->ss.p);
     act->dim_cap = in_dim;
-    if (type == TYPE_Q4_K && n_tokens >= ACT_H_ROWS) {
+    if (f16) {
         act->dt_pitch = (n_tokens + 3) / 4 * 4;
         if ((rc = ensure(ctx, ctx->sh, (size_t)n_tokens * in_dim * 2))) return rc;
         if ((rc = ensure(ctx, ctx->shs, (size_t)n_tokens * (in_dim / 16) * 2))) return rc;
@@ -325,11 +325,6 @@ int matmul_device(ob_ctx *ctx, const float *x_dev, uint32_t n_tokens, const ob_w
     }
     // one token, Q8_0: the product kernel quantizes the row in its prologue (one launch instead of two)
     const bool fused_q8 = n_tokens == 1 && w->w.type == TYPE_Q8_0;
-    ActBuf act{};
-    if (!fused_q8) {
-        int rc = quantize_for(ctx, x_dev, n_tokens, w->w.in_dim, w->w.type, &act, st);
-        if (rc) return rc;
-    }
     GemvArgs a{};
     a.x_f32 = fused_q8 ? x_dev : nullptr;
     a.n_seg = 1;
@@ -342,11 +337,15 @@ int matmul_device(ob_ctx *ctx, const float *x_dev, uint32_t n_tokens, const ob_w
     a.seg[0].y = y_dev;
     a.seg[0].y_stride = a.seg[0].w.out_dim;
     a.seg[0].epilogue = EPI_STORE;
-    a.act = act;
     a.n_tokens = n_tokens;
     a.gemm_order = !decode && n_tokens > 1;
     a.isum_out = isum_out;
     a.imin_out = imin_out;
+    if (!fused_q8) {
+        a.act.dim_cap = w->w.in_dim;
+        int rc = quantize_for(ctx, x_dev, n_tokens, w->w.in_dim, w->w.type, gemv_reads_f16(a, ctx->sm_count), &a.act, st);
+        if (rc) return rc;
+    }
     ctx->launches += launch_gemv(a, ctx->sm_count, st);
     return OB_OK;
 }
@@ -534,7 +533,7 @@ int ob_quantize_act(ob_ctx *ctx, const float *x, uint32_t n, int per_256, int8_t
     if ((rc = ensure(ctx, ctx->sx, (size_t)n * 4))) return rc;
     OB_CUDA(ctx, cudaMemcpyAsync(ctx->sx.p, x, (size_t)n * 4, cudaMemcpyHostToDevice, ctx->stream));
     ActBuf act;
-    if ((rc = quantize_for(ctx, static_cast<float *>(ctx->sx.p), 1, n, per_256 ? TYPE_Q4_K : TYPE_Q8_0, &act, ctx->stream))) return rc;
+    if ((rc = quantize_for(ctx, static_cast<float *>(ctx->sx.p), 1, n, per_256 ? TYPE_Q4_K : TYPE_Q8_0, false, &act, ctx->stream))) return rc;
     std::vector<int16_t> s16(n / 16);
     OB_CUDA(ctx, cudaMemcpyAsync(q, act.q, n, cudaMemcpyDeviceToHost, ctx->stream));
     OB_CUDA(ctx, cudaMemcpyAsync(d, act.d, (size_t)(n / grp) * 4, cudaMemcpyDeviceToHost, ctx->stream));

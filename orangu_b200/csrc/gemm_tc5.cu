@@ -656,7 +656,7 @@ bool gemm_tc5_supported(const GemvArgs &a) {
     if (type == TYPE_Q8_0) {
         if (in_dim % 128 || a.act.dim_cap % 128) return false;
     } else if (type == TYPE_Q4_K) {
-        if (in_dim % 256 || in_dim / 256 > 256 || !a.act.h || a.act.dim_cap % 256) return false;
+        if (in_dim % 256 || in_dim / 256 > 256 || a.act.dim_cap % 256) return false;
         for (int s = 0; s < a.n_seg; ++s)
             if (!a.seg[s].wide || !a.seg[s].wide->flags) return false;
     } else {
@@ -747,6 +747,7 @@ static KqChoice choose_q4k(const GemvArgs &a, int sm_count) {
 double gemm_tc5_q4k_us(const GemvArgs &a, int sm_count) { return choose_q4k(a, std::max(1, sm_count)).us; }
 
 static uint32_t launch_q4k(const GemvArgs &a, int sm_count, cudaStream_t st) {
+    if (!a.act.h) return 0;
     const KqChoice c = choose_q4k(a, std::max(1, sm_count));
     if (a.gemm_order && !c.two) {
         switch (c.n) {

@@ -438,6 +438,32 @@ size_t gemv_smem_bytes(uint32_t type, uint32_t in_dim, uint32_t tile_tokens, boo
     return smem_plan(type, in_dim, tile_tokens, gemm_order).total;
 }
 
+// Whether the few-token kernel takes a product; tc5: the tcgen05 tiles could.
+static bool takes_few(const GemvArgs &a, bool tc5, int sm_count) {
+    if (!gemm_few_supported(a)) return false;
+    // A few tokens (gemm_few.cu), against tcgen05 tiles by what both take.  Q6_K has none, and its 64-row tiles (gemm_mma.cu) overtake at
+    // 14336 x 4096 with 9 tokens (33 us against 35), at 32768 x 4096 with 17 (72 against 108), at 4096 x 14336 with 33 (86 against 88).
+    // The dp4a kernel below is ahead with 2 or 3 tokens where tiles go round several times.  Us, dp4a and gemm_few, rows of 4096:
+    //   Q4_K, 2 tokens, prefill order: 6144 rows 16.5 and 16.2, 8192 16.8 and 18.6, 14336 22.7 and 25.9, 28672 33.0 and 41.2
+    //   Q4_K, 3 tokens: 8192 18.6 and 18.6, 14336 25.3 and 26.5, 28672 38.6 and 41.2 (but 14336 rows of 8192 43.2 and 37.0)
+    //   Q6_K, 2 tokens, decode order: 9472 18.8 and 18.6, 12288 22.6 and 24.5, 28672 37.1 and 40.4; prefill order: 24.7 and 22.9 (14336)
+    //   Q6_K, 3 tokens: 9600 22.7 and 18.6, 14336 27.0 and 22.9, 28672 41.3 and 37.1 (decode order 27.3 and 25.6, 41.5 and 41.0)
+    uint32_t rows = 0;
+    for (int s = 0; s < a.n_seg; ++s) rows += a.seg[s].w.out_dim;
+    const uint32_t round = 16 * 2 * (uint32_t)sm_count;  // rows that all SMs take at once
+    const bool rounds = rows > 2 * round;
+    bool dp4a;
+    if (a.seg[0].w.type == TYPE_Q4_K) dp4a = a.n_tokens == 2 ? 2 * rows > 3 * round : a.n_tokens == 3 && rounds;
+    else dp4a = a.n_tokens == 2 && rounds && !a.gemm_order;
+    if (dp4a) return false;
+    if (tc5) return gemm_few_us(a) < gemm_tc5_q4k_us(a, sm_count);
+    return a.n_tokens <= (rounds ? 8u : 16u) || (a.n_tokens <= 32 && rows <= 8192);
+}
+
+bool gemv_reads_f16(const GemvArgs &a, int sm_count) {
+    return a.n_seg > 0 && a.seg[0].w.type == TYPE_Q4_K && gemm_tc5_supported(a) && !takes_few(a, true, sm_count);
+}
+
 uint32_t launch_gemv(const GemvArgs &a, int sm_count, cudaStream_t st) {
     if (a.n_tokens == 0 || a.n_seg == 0) return 0;
     if (a.seg[0].w.type == TYPE_Q5_K) {  // its own kernel, both orders (q5k.cu)
@@ -446,27 +472,7 @@ uint32_t launch_gemv(const GemvArgs &a, int sm_count, cudaStream_t st) {
     }
     static const bool use_mma = [] { const char *e = getenv("OB_MMA"); return !(e && e[0] == '0' && e[1] == 0); }();
     const bool tc5 = gemm_tc5_supported(a);
-    if (gemm_few_supported(a)) {
-        // A few tokens (gemm_few.cu), against tcgen05 tiles by what both take.  Q6_K has none, and its 64-row tiles (gemm_mma.cu) overtake at
-        // 14336 x 4096 with 9 tokens (33 us against 35), at 32768 x 4096 with 17 (72 against 108), at 4096 x 14336 with 33 (86 against 88).
-        // The dp4a kernel below is ahead with 2 or 3 tokens where tiles go round several times.  Us, dp4a and gemm_few, rows of 4096:
-        //   Q4_K, 2 tokens, prefill order: 6144 rows 16.5 and 16.2, 8192 16.8 and 18.6, 14336 22.7 and 25.9, 28672 33.0 and 41.2
-        //   Q4_K, 3 tokens: 8192 18.6 and 18.6, 14336 25.3 and 26.5, 28672 38.6 and 41.2 (but 14336 rows of 8192 43.2 and 37.0)
-        //   Q6_K, 2 tokens, decode order: 9472 18.8 and 18.6, 12288 22.6 and 24.5, 28672 37.1 and 40.4; prefill order: 24.7 and 22.9 (14336)
-        //   Q6_K, 3 tokens: 9600 22.7 and 18.6, 14336 27.0 and 22.9, 28672 41.3 and 37.1 (decode order 27.3 and 25.6, 41.5 and 41.0)
-        uint32_t rows = 0;
-        for (int s = 0; s < a.n_seg; ++s) rows += a.seg[s].w.out_dim;
-        const uint32_t round = 16 * 2 * (uint32_t)sm_count;  // rows that all SMs take at once
-        const bool rounds = rows > 2 * round;
-        bool dp4a;
-        if (a.seg[0].w.type == TYPE_Q4_K) dp4a = a.n_tokens == 2 ? 2 * rows > 3 * round : a.n_tokens == 3 && rounds;
-        else dp4a = a.n_tokens == 2 && rounds && !a.gemm_order;
-        bool few;
-        if (dp4a) few = false;
-        else if (tc5) few = gemm_few_us(a) < gemm_tc5_q4k_us(a, sm_count);
-        else few = a.n_tokens <= (rounds ? 8u : 16u) || (a.n_tokens <= 32 && rows <= 8192);
-        if (few && launch_gemm_few(a, sm_count, st)) return 1;
-    }
+    if (takes_few(a, tc5, sm_count) && launch_gemm_few(a, sm_count, st)) return 1;
     if (tc5) {  // many tokens: tcgen05 tiles (gemm_tc5.cu)
         if (const uint32_t n = launch_gemm_tc5(a, sm_count, st)) return n;
     }

@@ -27,8 +27,8 @@ struct ActBuf {
     float *d = nullptr;      // [rows][dim/group]
     int16_t *sums = nullptr; // [rows][dim/16]
     uint32_t dim_cap = 0;    // row pitch in elements
-    // per-256 only, for the tcgen05 products of Q4_K (gemm_tc5.cu); written for ACT_H_ROWS rows or more
-    __half *h = nullptr;     // [rows][dim] the codes as f16, elements 0 2 1 3 of every four
+    // per-256 only, for the tcgen05 products of Q4_K (gemm_tc5.cu): where one reads them (gemv_reads_f16), which takes ACT_H_ROWS rows
+    __half *h = nullptr;     // [rows][dim] the codes as f16, elements 0 2 1 3 of every four; null: none of the three is written or read
     __half *hs = nullptr;    // [rows][dim/16] per 256: the eight sums of 32 as lo + 64 hi, the lows (-32 .. 31), then the highs
     float *dt = nullptr;     // [dim/256][dt_pitch] d with the rows side by side
     uint32_t dt_pitch = 0;   // a multiple of 4
@@ -66,6 +66,8 @@ struct GemvArgs {
     int32_t *isum_out;     // optional debug capture (single segment, token 0): [out_dim][nb]
     int32_t *imin_out;
 };
+// Whether the product reads the f16 codes, sums and scales of `act` (act.dim_cap has to be set for that, nothing else of act).
+OB_QUANT bool gemv_reads_f16(const GemvArgs &a, int sm_count);
 OB_QUANT uint32_t launch_gemv(const GemvArgs &a, int sm_count, cudaStream_t st);  // kernels launched
 OB_QUANT size_t gemv_smem_bytes(uint32_t type, uint32_t in_dim, uint32_t tile_tokens, bool gemm_order);
 
@@ -84,8 +86,8 @@ OB_QUANT bool gemm_mma_supported(const GemvArgs &a);
 OB_QUANT void launch_gemm_mma(const GemvArgs &a, int sm_count, cudaStream_t st);
 
 // ---- gemm_tc5.cu: many-token products on tcgen05 tensor cores with TMEM accumulators, TMA-fed (Q8_0 16 tokens or more, Q4_K ACT_H_ROWS)
-OB_QUANT bool gemm_tc5_supported(const GemvArgs &a);
-OB_QUANT uint32_t launch_gemm_tc5(const GemvArgs &a, int sm_count, cudaStream_t st);  // kernels launched; 0: a tensor map could not be made, or a row is too long
+OB_QUANT bool gemm_tc5_supported(const GemvArgs &a);  // whatever act.h is
+OB_QUANT uint32_t launch_gemm_tc5(const GemvArgs &a, int sm_count, cudaStream_t st);  // kernels launched; 0: a tensor map could not be made, a row is too long, or Q4_K without act.h
 OB_QUANT double gemm_tc5_q4k_us(const GemvArgs &a, int sm_count);  // about how long it takes
 OB_QUANT int gemm_tc5_take_status();  // 1 when a bounded wait inside one of these kernels ran out since the last call
 OB_QUANT void gemm_tc5_mark_launched();  // a replayed graph may have run one of them

@@ -10,6 +10,7 @@
 #include <cmath>
 #include <functional>
 #include <map>
+#include <tuple>
 #include <vector>
 
 #include "model.h"
@@ -44,7 +45,8 @@ __global__ void __launch_bounds__(256) copy_pages_kernel(__half *k_pool, __half 
 
 namespace {
 
-int alloc_act(ob_model *m, ActPair *a, uint32_t rows, uint32_t dim) {
+// f16: some product of these activations is of a Q4_K weight
+int alloc_act(ob_model *m, ActPair *a, uint32_t rows, uint32_t dim, bool f16) {
     int rc;
     for (ActBuf *b : {&a->k, &a->flat}) {
         const uint32_t grp = b == &a->k ? 256u : 32u;
@@ -53,7 +55,7 @@ int alloc_act(ob_model *m, ActPair *a, uint32_t rows, uint32_t dim) {
         if ((rc = dev_alloc(m, &b->sums, (size_t)rows * (dim / 16)))) return rc;
         b->dim_cap = dim;
     }
-    if (rows >= ACT_H_ROWS && dim % 256 == 0) {
+    if (f16 && rows >= ACT_H_ROWS) {
         a->k.dt_pitch = (rows + 3) / 4 * 4;
         if ((rc = dev_alloc(m, &a->k.h, (size_t)rows * dim))) return rc;
         if ((rc = dev_alloc(m, &a->k.hs, (size_t)rows * (dim / 16)))) return rc;
@@ -77,17 +79,6 @@ int slice_weight(ob_model *m, const ob_matrix_desc &d, uint32_t row0, uint32_t n
     return make_weight(m->ctx, d.data, rb, d.ggml_type, d.in_dim, d.out_dim, row0, n_rows, col0, n_cols, out);
 }
 
-bool needs_k(std::initializer_list<const ob_weight *> ws) {
-    for (auto w : ws)
-        if (w->w.type != TYPE_Q8_0) return true;
-    return false;
-}
-bool needs_flat(std::initializer_list<const ob_weight *> ws) {
-    for (auto w : ws)
-        if (w->w.type == TYPE_Q8_0) return true;
-    return false;
-}
-
 const ActBuf &act_for(const ActPair &p, const ob_weight *w) { return w->w.type == TYPE_Q8_0 ? p.flat : p.k; }
 
 // Products that share one input: one launch per distinct weight type.
@@ -98,9 +89,14 @@ struct ProductOut {
     const float *residual;
 };
 
-void run_products(ob_model *m, const ActPair &act, std::initializer_list<ProductOut> outs, uint32_t n_tokens, bool gemm_order, cudaStream_t st) {
+// Quantizes x (see ActSource) as the products of `outs` read it, then runs them.
+void run_products(ob_model *m, int source, const float *x, const float *aux, uint32_t dim, const ActPair &act, std::initializer_list<ProductOut> outs,
+                  uint32_t n_tokens, bool gemm_order, cudaStream_t st) {
     std::vector<ProductOut> v(outs);
     std::vector<bool> done(v.size(), false);
+    std::vector<GemvArgs> products;
+    QuantArgs qa{};
+    bool f16 = false;
     for (size_t i = 0; i < v.size(); ++i) {
         if (done[i]) continue;
         GemvArgs a{};
@@ -118,22 +114,20 @@ void run_products(ob_model *m, const ActPair &act, std::initializer_list<Product
             s.epilogue = v[j].residual ? EPI_ADD_RESIDUAL : EPI_STORE;
             done[j] = true;
         }
-        m->ctx->launches += launch_gemv(a, m->ctx->sm_count, st);
+        if (!gemv_reads_f16(a, m->ctx->sm_count)) a.act.h = nullptr;
+        f16 = f16 || a.act.h;
+        (a.seg[0].w.type == TYPE_Q8_0 ? qa.flat : qa.k) = a.act;
+        products.push_back(a);
     }
-}
-
-void quantize_into(ob_model *m, int source, const float *x, const float *aux, uint32_t rows, uint32_t dim, const ActPair &dst, bool want_k,
-                   bool want_flat, cudaStream_t st) {
-    QuantArgs qa{};
     qa.x = x;
     qa.aux = aux;
     qa.eps = m->cfg.rms_eps;
-    qa.n_rows = rows;
+    qa.n_rows = n_tokens;
     qa.dim = dim;
-    if (want_k) qa.k = dst.k;
-    if (want_flat) qa.flat = dst.flat;
+    if (f16) qa.k.h = act.k.h;  // (one of the products that share the codes)
     launch_quantize(source, qa, st);
     m->ctx->launches++;
+    for (const GemvArgs &a : products) m->ctx->launches += launch_gemv(a, m->ctx->sm_count, st);
 }
 
 int check_peer(ob_model *m);
@@ -553,8 +547,8 @@ void enqueue_step(ob_model *m, uint32_t T, bool gemm_order, uint32_t logit_row0,
             m->ctx->launches++;
             pending_exchange = false;
         }
-        quantize_into(m, ACT_RMSNORM, m->x, L.attn_norm, T, n_embd, m->act_embd, needs_k({L.wq, L.wk, L.wv}), needs_flat({L.wq, L.wk, L.wv}), st);
-        run_products(m, m->act_embd, {{L.wq, m->q, q_dim, nullptr}, {L.wk, m->k, kv_dim, nullptr}, {L.wv, m->v, kv_dim, nullptr}}, T, gemm_order, st);
+        run_products(m, ACT_RMSNORM, m->x, L.attn_norm, n_embd, m->act_embd,
+                     {{L.wq, m->q, q_dim, nullptr}, {L.wk, m->k, kv_dim, nullptr}, {L.wv, m->v, kv_dim, nullptr}}, T, gemm_order, st);
 
         RopeKvArgs rk{};
         rk.q = m->q;
@@ -582,21 +576,18 @@ void enqueue_step(ob_model *m, uint32_t T, bool gemm_order, uint32_t logit_row0,
 
         run_attention(m, li, T, exact_attn, pos_bound, nullptr, d_tables, d_npos, st, gemm_order);
 
-        quantize_into(m, ACT_PLAIN, m->attn, nullptr, T, q_dim, m->act_attn, needs_k({L.wo}), needs_flat({L.wo}), st);
         if (!tp) {
-            run_products(m, m->act_attn, {{L.wo, m->x, n_embd, m->x}}, T, gemm_order, st);
+            run_products(m, ACT_PLAIN, m->attn, nullptr, q_dim, m->act_attn, {{L.wo, m->x, n_embd, m->x}}, T, gemm_order, st);
         } else {
-            run_products(m, m->act_attn, {{L.wo, m->proj, n_embd, nullptr}}, T, gemm_order, st);
+            run_products(m, ACT_PLAIN, m->attn, nullptr, q_dim, m->act_attn, {{L.wo, m->proj, n_embd, nullptr}}, T, gemm_order, st);
             reduce_rows(T);
         }
 
-        quantize_into(m, ACT_RMSNORM, m->x, L.ffn_norm, T, n_embd, m->act_embd, needs_k({L.gate, L.up}), needs_flat({L.gate, L.up}), st);
-        run_products(m, m->act_embd, {{L.gate, m->gate, n_ff, nullptr}, {L.up, m->up, n_ff, nullptr}}, T, gemm_order, st);
-        quantize_into(m, ACT_SWIGLU, m->gate, m->up, T, n_ff, m->act_ff, needs_k({L.down}), needs_flat({L.down}), st);
+        run_products(m, ACT_RMSNORM, m->x, L.ffn_norm, n_embd, m->act_embd, {{L.gate, m->gate, n_ff, nullptr}, {L.up, m->up, n_ff, nullptr}}, T, gemm_order, st);
         if (!tp) {
-            run_products(m, m->act_ff, {{L.down, m->x, n_embd, m->x}}, T, gemm_order, st);
+            run_products(m, ACT_SWIGLU, m->gate, m->up, n_ff, m->act_ff, {{L.down, m->x, n_embd, m->x}}, T, gemm_order, st);
         } else {
-            run_products(m, m->act_ff, {{L.down, m->proj, n_embd, nullptr}}, T, gemm_order, st);
+            run_products(m, ACT_SWIGLU, m->gate, m->up, n_ff, m->act_ff, {{L.down, m->proj, n_embd, nullptr}}, T, gemm_order, st);
             reduce_rows(T);
         }
     }
@@ -642,9 +633,8 @@ void enqueue_step(ob_model *m, uint32_t T, bool gemm_order, uint32_t logit_row0,
     }
     if (n_logit_rows && !(n_logit_rows == 1 && stream && m->stream_ok && k_type(m->output))) {
         const float *xl = m->x + (size_t)logit_row0 * n_embd;
-        quantize_into(m, ACT_RMSNORM, xl, m->output_norm, n_logit_rows, n_embd, m->act_embd, needs_k({m->output}), needs_flat({m->output}), st);
         // Always the single-token kernel: forward() projects one row (llama.rs:1026-1030).
-        run_products(m, m->act_embd, {{m->output, m->logits + m->vocab0, c.n_vocab, nullptr}}, n_logit_rows, false, st);
+        run_products(m, ACT_RMSNORM, xl, m->output_norm, n_embd, m->act_embd, {{m->output, m->logits + m->vocab0, c.n_vocab, nullptr}}, n_logit_rows, false, st);
         finish_logits(n_logit_rows);
     }
     m->last_T = T;
@@ -825,9 +815,16 @@ int ob_model_create(ob_ctx *ctx, const ob_model_desc *desc, ob_model **out) {
     if ((rc = dev_alloc(m, &m->up, (size_t)T * m->n_ff_l))) return bail(rc);
     if ((rc = dev_alloc(m, &m->proj, (size_t)T * c.n_embd))) return bail(rc);
     if ((rc = dev_alloc(m, &m->logits, (size_t)T * c.n_vocab))) return bail(rc);
-    if ((rc = alloc_act(m, &m->act_embd, T, c.n_embd))) return bail(rc);
-    if ((rc = alloc_act(m, &m->act_attn, T, q_dim))) return bail(rc);
-    if ((rc = alloc_act(m, &m->act_ff, T, m->n_ff_l))) return bail(rc);
+    auto any_q4k = [m](std::initializer_list<ob_weight *LayerDev::*> ws) {
+        for (const LayerDev &L : m->layers)
+            for (auto w : ws)
+                if ((L.*w)->w.type == TYPE_Q4_K) return true;
+        return false;
+    };
+    const bool embd_q4k = m->output->w.type == TYPE_Q4_K || any_q4k({&LayerDev::wq, &LayerDev::wk, &LayerDev::wv, &LayerDev::gate, &LayerDev::up});
+    if ((rc = alloc_act(m, &m->act_embd, T, c.n_embd, embd_q4k))) return bail(rc);
+    if ((rc = alloc_act(m, &m->act_attn, T, q_dim, any_q4k({&LayerDev::wo})))) return bail(rc);
+    if ((rc = alloc_act(m, &m->act_ff, T, m->n_ff_l, any_q4k({&LayerDev::down})))) return bail(rc);
     m->max_splits = std::max(1u, std::min(64u, (m->cfg.max_seq_len + 63) / 64));
     {   // rows * pick_splits(rows) never exceeds 4 * SMs + rows; the fused kernel's own rule (run_attention) takes up to
         // four splits per row however many rows there are
@@ -1113,9 +1110,18 @@ int ob_profile_gemv(ob_model *m, uint32_t ggml_type, uint32_t variant, uint32_t 
     OB_CUDA(ctx, cudaMemsetAsync(m->x, 0, (size_t)m->cfg.n_embd * 4, st));
     OB_CUDA(ctx, cudaMemsetAsync(m->attn, 0, (size_t)m->n_head_l * m->cfg.head_dim * 4, st));
     OB_CUDA(ctx, cudaMemsetAsync(m->gate, 0, (size_t)m->n_ff_l * 4, st));
-    quantize_into(m, ACT_PLAIN, m->x, nullptr, 1, m->cfg.n_embd, m->act_embd, true, true, st);
-    quantize_into(m, ACT_PLAIN, m->attn, nullptr, 1, m->n_head_l * m->cfg.head_dim, m->act_attn, true, true, st);
-    quantize_into(m, ACT_PLAIN, m->gate, nullptr, 1, m->n_ff_l, m->act_ff, true, true, st);
+    for (const auto &[x, dim, act] : {std::make_tuple(m->x, m->cfg.n_embd, &m->act_embd), std::make_tuple(m->attn, m->n_head_l * m->cfg.head_dim, &m->act_attn),
+                                      std::make_tuple(m->gate, m->n_ff_l, &m->act_ff)}) {
+        QuantArgs qa{};
+        qa.x = x;
+        qa.n_rows = 1;
+        qa.dim = dim;
+        qa.k = act->k;
+        qa.k.h = nullptr;
+        qa.flat = act->flat;
+        launch_quantize(ACT_PLAIN, qa, st);
+        ctx->launches++;
+    }
     uint64_t bytes = 0;
     uint32_t launches = 0;
     for (uint32_t it = 0; it <= iters; ++it) {  // pass 0 is a warm-up

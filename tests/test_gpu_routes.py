@@ -50,6 +50,23 @@ def test_two_and_three_tokens(backend, t, rows, n, prefill, decode):
         assert_bit_equal(run(x, n, w), oracle(x, n, w.raw, t, cols, rows), "products")
 
 
+def test_f16_codes_are_held_only_for_q4k_weights(backend):
+    """The tiles of Q4_K read activations in a form of their own, 2.2 bytes an entry; a model without Q4_K weights holds none of it."""
+    import torch
+
+    cfg = dict(n_vocab=256, n_embd=256, n_layer=1, n_head=4, n_head_kv=2, head_dim=64, n_ff=8192, rope_freq_base=10000.0, rms_eps=1e-5)
+    names = ("token_embd", "output", "attn_q", "attn_k", "attn_v", "attn_output", "ffn_gate", "ffn_up", "ffn_down")
+    used = {}
+    for t in (Q4_K, Q6_K):
+        tensors = synth.model_tensors(cfg, seed=3, types={name: t for name in names})
+        before = torch.cuda.mem_get_info()[0]
+        model = LlamaModel(backend, cfg, tensors, max_seq_len=4096, max_batch_tokens=4096, exact_attention_max_pos=64)
+        used[t] = before - torch.cuda.mem_get_info()[0]
+        model.close()
+    entries = 4096 * (256 + 256 + 8192)
+    assert used[Q4_K] - used[Q6_K] > 1.9 * entries, used  # (weights of Q6_K are the larger, by 4.5 MB)
+
+
 @pytest.mark.parametrize("t,n_seq", [(Q4_K, 16), (Q8_0, 16)])
 def test_a_wait_that_ran_out_in_a_replayed_step_is_reported(backend, t, n_seq):
     """The steps of a decode loop are captured at its first call and only replayed afterwards; the status that their products leave is read
