@@ -1,18 +1,10 @@
-// Many-token products on the fifth-generation tensor cores: tcgen05.mma (kind::i8) with accumulators in tensor memory,
-// operands brought into shared memory by TMA (cp.async.bulk.tensor, no multicast: every tensor map covers this GPU's own
-// memory and every CTA fetches its own tiles).
+// Many-token products on the fifth-generation tensor cores: tcgen05.mma with accumulators in tensor memory, operands brought into shared
+// memory by TMA (cp.async.bulk.tensor, no multicast: every tensor map covers this GPU's own memory and every CTA fetches its own tiles).
+// Q8_0 as int8 products, Q4_K as f16 products of whole numbers; the arithmetic is the reference's, so the results equal the CPU's bit for
+// bit at any batch size.
 //
-// The arithmetic is the reference's, so the results equal the CPU's bit for bit at any batch size:
-//   Q8_0 (engine/vecdot.rs:2598-2629 flat GEMM, :2829-2838 decode): acc += (ad_b * s_b) * (f32)dot32_b per block of 32, in
-//   block order.  The int8 codes of a row are already a K-major int8 matrix, so TMA loads them straight into the
-//   128-byte-swizzled operand layout.  One fp32 rounding per 32 elements means every K = 32 step needs its own integer
-//   result: each tcgen05.mma (M = 128 rows, N = 64 tokens, K = 32) writes a fresh accumulator, four per pipeline step in
-//   one half of tensor memory while the epilogue warps drain the other half (tcgen05.ld), scale and accumulate in fp32.
-//
-// Roles in a CTA of ten warps: warps 0-7 epilogue (warp w reads the 32 tensor-memory lanes of quadrant w % 4, token columns
-// 32 * (w / 4) ..), warp 8 lane 0 issues the TMA loads, warp 9 allocates tensor memory and its lane 0 issues the MMAs.
-// Stages and accumulator halves are handed over through mbarriers; every wait is bounded -- a wait that runs out sets a
-// status word, makes all roles leave their loops, and the CTA frees its tensor memory and returns.
+// Stages and accumulators are handed over through mbarriers; every wait is bounded -- a wait that runs out sets a status word, all roles
+// end, nothing more is stored, and the CTA frees its tensor memory and returns.
 #include "common.cuh"
 #include "kernels.h"
 #include "packed.cuh"
@@ -41,6 +33,14 @@ __host__ __device__ constexpr uint32_t umma_idesc_i8(uint32_t a_signed, uint32_t
 }
 
 // ---- Q8_0 ------------------------------------------------------------------------------------------------------------
+// engine/vecdot.rs:2598-2629 (flat GEMM), :2829-2838 (decode): acc += (ad_b * s_b) * (f32)dot32_b per block of 32, in block order.  The int8
+// codes of a row are already a K-major int8 matrix, so TMA loads them straight into the 128-byte-swizzled operand layout.  One fp32 rounding
+// per 32 elements means every K = 32 step needs its own integer result: each tcgen05.mma kind::i8 (M = 128 rows, N = 64 tokens, K = 32) writes
+// a fresh accumulator, four per pipeline step in one half of tensor memory while the epilogue warps drain the other half (tcgen05.ld), scale
+// and accumulate in fp32.
+//
+// Roles in a CTA of ten warps: warps 0-7 epilogue (warp w reads the 32 tensor-memory lanes of quadrant w % 4, token columns 32 * (w / 4) ..),
+// warp 8 lane 0 issues the TMA loads, warp 9 allocates tensor memory and its lane 0 issues the MMAs.
 constexpr int Q8_STAGES = 4;
 constexpr uint32_t Q8_A_BYTES = TC_M * 128, Q8_B_BYTES = TC_N * 128, Q8_XD_BYTES = TC_N * 16;
 struct Q8Smem {  // offsets from the 1024-byte aligned base
@@ -190,9 +190,9 @@ gemm_tc5_q8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 // (0, 2, 1, 3); the quantizer writes activations in that order.
 //
 // The form before had byte planes of the weights' scale digits in shared memory, int8 products and two or three accumulators to read
-// back: 14336 x 4096 with 512 tokens 213 us in prefill order (now 132), 4096 x 14336 with 64 tokens 70 us in decode order on mma.sync
-// tiles (now 55).  What bounds this form is instruction issue: five warps share a scheduler, and a super-block's expansion, epilogue and
-// product issue are some 250 instructions each.
+// back: 14336 x 4096 with 509 tokens 213 us in prefill order (now 130), 4096 x 14336 with 64 tokens 70 us in decode order on mma.sync
+// tiles (now 52).  What bounds this form is the chain of its warps, five to a scheduler: 53 % of the issue slots are used and the tensor pipe
+// is busy for 29 % of the time, at 320 instructions a warp and super-block, both sweeps of the prefill order together.
 constexpr int KQ_EPI_WARPS = 8, KQ_EXP_WARPS = 8, KQ_TMA_WARP = 16, KQ_MMA_WARP = 17, KQ_THREADS = 19 * 32;
 constexpr uint32_t KQ_RAW_BYTES = TC_M * 144, KQ_A_COLS = 128;
 // TWO: the halves of a super-block have accumulators of their own (matrices with many wide rows).

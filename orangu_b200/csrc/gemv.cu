@@ -450,7 +450,7 @@ static bool takes_few(const GemvArgs &a, bool tc5, int sm_count) {
     //   Q6_K, 3 tokens: 9600 22.7 and 18.6, 14336 27.0 and 22.9, 28672 41.3 and 37.1 (decode order 27.3 and 25.6, 41.5 and 41.0)
     uint32_t rows = 0;
     for (int s = 0; s < a.n_seg; ++s) rows += a.seg[s].w.out_dim;
-    const uint32_t round = 16 * 2 * (uint32_t)sm_count;  // rows that all SMs take at once
+    const uint32_t round = 16 * 2 * (uint32_t)sm_count;  // two tiles of 16 rows an SM, 4736 rows of 148
     const bool rounds = rows > 2 * round;
     bool dp4a;
     if (a.seg[0].w.type == TYPE_Q4_K) dp4a = a.n_tokens == 2 ? 2 * rows > 3 * round : a.n_tokens == 3 && rounds;

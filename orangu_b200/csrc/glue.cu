@@ -81,11 +81,9 @@ __global__ void __launch_bounds__(256) rope_kv_kernel(RopeKvArgs a) {
     }
 }
 
-// The same step for the Qwen-style variants: bias, per-head RMSNorm, either pairing.  One CTA per token; the rows live in
-// shared memory between the steps.  The per-head sum of squares is added left to right by one thread per head, as
-// rmsnorm_inplace does it (engine/tensor.rs:691-700) -- head_dim is 64..256, so the sequential loop is short.
-// A warp per head (of q, k or v) of a token.  The norm's sum goes left to right: its squares are made side by side and every lane adds
-// them up from shared memory, 4 clocks an element (one thread a head in a CTA a token had all heads in one bank: 21.6 us for 8 tokens of
+// The same step for the Qwen-style variants: bias, per-head RMSNorm, either pairing.  A warp per head (of q, k or v) of a token; the head
+// lives in shared memory between the steps.  The norm's sum goes left to right, as rmsnorm_inplace does it (engine/tensor.rs:691-700): its
+// squares are made side by side and every lane adds them up from shared memory, 4 clocks an element (one thread a head in a CTA a token had all heads in one bank: 21.6 us for 8 tokens of
 // 40 heads x 128).
 constexpr int QP_WARPS = 4;
 __global__ void __launch_bounds__(QP_WARPS * 32) qkv_post_kernel(RopeKvArgs a) {

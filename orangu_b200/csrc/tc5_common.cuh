@@ -120,8 +120,7 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
 template <int C>
 __device__ __forceinline__ void tmem_ldn(uint32_t taddr, uint32_t (&r)[C]) {
     if constexpr (C == 8) tmem_ld8(taddr, r);
-    else if constexpr (C == 16) tmem_ld16(taddr, r);
-    else tmem_ld32(taddr, r);
+    else tmem_ld16(taddr, r);
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 

@@ -287,8 +287,8 @@ def test_8b_shape_two_layers_bit_exact(backend):
 
 
 def test_8b_shape_prefill_chunk_of_300_tokens_is_bit_exact(backend):
-    """One 300-token chunk at the 8B widths: three 128-token tiles, where the tcgen05 kernel serves ffn_gate and ffn_up from one
-    launch (2 x 336 CTAs are five waves of 148 together, six apart) and attn_q / attn_output / ffn_down from their own."""
+    """One 300-token chunk at the 8B widths: tiles of 96 and of 64 tokens on the tcgen05 kernel, the last one ragged, where attn_q and attn_k, and
+    ffn_gate and ffn_up, share a launch."""
     cfg = dict(synth.CONFIGS["8b"])
     cfg["n_layer"] = 1
     cfg["n_vocab"] = 4096

@@ -19,13 +19,33 @@ def both_orders(backend, w, x, n):
     assert_bit_equal(backend.matmul_decode(x, n, w).reshape(-1), O.matmul_decode(x, n, w.raw, *shape).reshape(-1), f"decode order, {n} tokens")
 
 
-# rows: not a multiple of 16 or 128; columns: one super-block, fewer than the warps that share a sum, more than a buffer of mins (16)
+# rows: not a multiple of 16 or 128; columns: one super-block, fewer than the warps that share a sum, more than a buffer of mins (16).  Mostly the
+# few-token kernel; tiles of 16 and 32 tokens from some 100 tokens on.
 @pytest.mark.parametrize("t", [Q4_K, Q6_K])
 @pytest.mark.parametrize("rows,cols", [(2100, 256), (1030, 768), (2100, 4608)])
 @pytest.mark.parametrize("n", [2, 7, 8, 9, 16, 17, 31, 33, 48, 49, 64, 65, 96, 97, 113, 129, 200])
 def test_products_at_the_edges_of_tiles(backend, t, rows, cols, n):
     w = QuantMatrix(synth.matrix(t, rows, cols, 5)["data"], t, cols, rows)
     both_orders(backend, w, synth.normal(n * cols, 6 + n), n)
+
+
+@pytest.mark.parametrize("few", [True, False])
+def test_sums_beyond_one_accumulator(backend, few):
+    """Rows whose every code is 15 and every scale 63 against activations of the largest code: halves of 15.4e6 and sums of 30.7e6, above
+    2^24; among rows of ordinary blocks, few of them or many.  (These sizes take the few-token kernel, whose sums are integers.)"""
+    rows, cols = 2100, 512
+    blocks = synth.matrix(Q4_K, rows, cols, 9)["data"].reshape(rows, -1, 144).copy()
+    full = np.r_[3:5, 130, 2099] if few else np.r_[3:5, 130, 700:900, 2099]
+    blocks[full, :, 4:12] = 0xff  # scales and mins 63, their upper bits too
+    blocks[full, :, 12:16] = 0xff
+    blocks[full, :, 16:] = 0xff
+    blocks[full[::2], :, 20:21] = 0x3e  # not all alike: odd sums as well
+    w = QuantMatrix(blocks.reshape(-1), Q4_K, cols, rows)
+    for n in (16, 40, 130):
+        x = np.random.default_rng(n).standard_normal((n, cols)).astype(np.float32)
+        x[::3] = 1.5
+        x[1::6] = np.where(np.arange(cols) % 7 == 0, -1.5, 1.5)
+        both_orders(backend, w, x.reshape(-1), n)
 
 
 # ---- the tcgen05 tiles of Q4_K

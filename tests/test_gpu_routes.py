@@ -36,7 +36,7 @@ def test_long_rows_of_many_tokens_take_the_tiles(backend):
     assert_bit_equal(backend.matmul(x, n, w), O.matmul(x, n, w.raw, Q4_K, cols, rows), "48 tokens")
 
 
-# 7104 and 9472 rows are one and a half times and twice what all SMs take at once; the kernels of prefill order, of decode order
+# 7104 and 9472 rows are three and four tiles of 16 rows an SM; the kernels of prefill order, of decode order
 @pytest.mark.parametrize("t,rows,n,prefill,decode", [
     (Q4_K, 7104, 2, "few", "few"), (Q4_K, 7105, 2, "gemv", "gemv"), (Q4_K, 9472, 3, "few", "few"), (Q4_K, 9473, 3, "gemv", "gemv"), (Q4_K, 9473, 4, "few", "few"),
     (Q6_K, 9472, 2, "few", "few"), (Q6_K, 9473, 2, "few", "gemv"), (Q6_K, 9473, 3, "few", "few")])
