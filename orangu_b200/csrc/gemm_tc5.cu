@@ -739,7 +739,9 @@ static KqChoice choose_q4k(const GemvArgs &a, int sm_count) {
         const uint32_t nb = a.seg[0].w.nb, raw = (w.n > 64 ? 3u : 4u) * KQ_RAW_BYTES, b = (w.n > 64 ? 2u : 3u) * w.n * (a.gemm_order ? 512u : 640u);
         if (raw + b + nb * w.n * 4 + 2048 > 227 * 1024) continue;
         const uint32_t tiles = rows * ((a.n_tokens + w.n - 1) / w.n), waves = (tiles + sm_count - 1) / sm_count;
-        const double us = 4.0 + (wide ? 3.0 : 0.0) + (best.two ? 1.3 : 1.0) * waves * nb * each;
+        // (with the quantizer, without wide rows, with a few, with halves apart: 4096 x 14336 with 64 tokens in prefill order 67.0, 66.3 and 74.1 us,
+        // 37838 x 2304 39.1, 40.0 and 43.2; 32 tokens in decode order 26.8, 28.8 and 28.8)
+        const double us = 4.0 + (wide ? 3.0 : 0.0) + (best.two ? 1.15 : 1.0) * waves * nb * each;
         if (us < best.us) best.us = us, best.n = w.n;
     }
     return best;
