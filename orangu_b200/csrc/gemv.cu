@@ -445,6 +445,7 @@ static bool takes_few(const GemvArgs &a, bool tc5, int sm_count) {
     // 14336 x 4096 with 9 tokens (33 us against 35), at 32768 x 4096 with 17 (72 against 108), at 4096 x 14336 with 33 (86 against 88).
     // The dp4a kernel below is ahead with 2 or 3 tokens where tiles go round several times.  Us, dp4a and gemm_few, rows of 4096:
     //   Q4_K, 2 tokens, prefill order: 6144 rows 16.5 and 16.2, 8192 16.8 and 18.6, 14336 22.7 and 25.9, 28672 33.0 and 41.2
+    //   and rows of 2048, 8192 of them: 13.3 and 14.5 in prefill order, 12.9 and 12.4 in decode order
     //   Q4_K, 3 tokens: 8192 18.6 and 18.6, 14336 25.3 and 26.5, 28672 38.6 and 41.2 (but 14336 rows of 8192 43.2 and 37.0)
     //   Q6_K, 2 tokens, decode order: 9472 18.8 and 18.6, 12288 22.6 and 24.5, 28672 37.1 and 40.4; prefill order: 24.7 and 22.9 (14336)
     //   Q6_K, 3 tokens: 9600 22.7 and 18.6, 14336 27.0 and 22.9, 28672 41.3 and 37.1 (decode order 27.3 and 25.6, 41.5 and 41.0)
@@ -453,7 +454,7 @@ static bool takes_few(const GemvArgs &a, bool tc5, int sm_count) {
     const uint32_t round = 16 * 2 * (uint32_t)sm_count;  // two tiles of 16 rows an SM, 4736 rows of 148
     const bool rounds = rows > 2 * round;
     bool dp4a;
-    if (a.seg[0].w.type == TYPE_Q4_K) dp4a = a.n_tokens == 2 ? 2 * rows > 3 * round : a.n_tokens == 3 && rounds;
+    if (a.seg[0].w.type == TYPE_Q4_K) dp4a = (rounds && a.n_tokens <= 3) || (a.n_tokens == 2 && 2 * rows > 3 * round && (a.gemm_order || a.seg[0].w.nb >= 16));
     else dp4a = a.n_tokens == 2 && rounds && !a.gemm_order;
     if (dp4a) return false;
     if (tc5) return gemm_few_us(a) < gemm_tc5_q4k_us(a, sm_count);

@@ -37,11 +37,11 @@ def test_long_rows_of_many_tokens_take_the_tiles(backend):
 
 
 # 7104 and 9472 rows are three and four tiles of 16 rows an SM; the kernels of prefill order, of decode order
-@pytest.mark.parametrize("t,rows,n,prefill,decode", [
-    (Q4_K, 7104, 2, "few", "few"), (Q4_K, 7105, 2, "gemv", "gemv"), (Q4_K, 9472, 3, "few", "few"), (Q4_K, 9473, 3, "gemv", "gemv"), (Q4_K, 9473, 4, "few", "few"),
-    (Q6_K, 9472, 2, "few", "few"), (Q6_K, 9473, 2, "few", "gemv"), (Q6_K, 9473, 3, "few", "few")])
-def test_two_and_three_tokens(backend, t, rows, n, prefill, decode):
-    cols = 768
+@pytest.mark.parametrize("t,rows,cols,n,prefill,decode", [
+    (Q4_K, 7104, 768, 2, "few", "few"), (Q4_K, 7105, 768, 2, "gemv", "few"), (Q4_K, 7105, 4096, 2, "gemv", "gemv"), (Q4_K, 9473, 768, 2, "gemv", "gemv"),
+    (Q4_K, 9472, 768, 3, "few", "few"), (Q4_K, 9473, 768, 3, "gemv", "gemv"), (Q4_K, 9473, 768, 4, "few", "few"),
+    (Q6_K, 9472, 768, 2, "few", "few"), (Q6_K, 9473, 768, 2, "few", "gemv"), (Q6_K, 9473, 768, 3, "few", "few")])
+def test_two_and_three_tokens(backend, t, rows, cols, n, prefill, decode):
     w = QuantMatrix(synth.matrix(t, rows, cols, 5)["data"], t, cols, rows)
     x = synth.normal(n * cols, 6)
     for run, want, oracle in ((backend.matmul, prefill, O.matmul), (backend.matmul_decode, decode, O.matmul_decode)):
